@@ -1147,6 +1147,7 @@ struct dqmc_handle {
     std::vector<void*> allocs;
     cudaStream_t st = nullptr;
     int nch = 0, maxN = 0, ltrot = 0, nst = 0, nwrap = 0, nnf_max = 0;
+    int team = 1;                    // CTAs per chain of the QR and Green's function kernels
     int started = 0;
     cudaGraphExec_t sweep_graph = nullptr;
     int graph_meas = -1;
@@ -1450,8 +1451,7 @@ extern "C" int dqmc_gpu_create(const dqmc_params* params, int n_params, int n_ch
         for (int c = 0; c < n_chains; ++c) v[c] = h->chains[c].dev;
         cudaMemcpy(h->d_chains, v.data(), sizeof(ChainDev) * n_chains, cudaMemcpyHostToDevice);
     }
-    set_stab_maxN(h->maxN);
-    if (h->proj) set_proj_maxN(h->maxN);
+    h->team = pick_team(n_chains);
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
     h->ctas_per_chain = std::max(1, std::min(h->maxN / 16, (2 * sms + n_chains - 1) / n_chains));
@@ -1606,9 +1606,9 @@ static void stab_0b(dqmc_handle* h, int n, int record) {
     tmark(h, DQMC_PROF_OTHER);
     launch_bmat(h, 2, m.wrap_step[(n - 1) * 2 + 1], m.wrap_step[(n - 1) * 2], 0);
     tmark(h, DQMC_PROF_BPROD);
-    launch_stab_slots(h->d_chains, h->nch, n - 1, spare, h->st);
+    launch_stab_slots(h->d_chains, h->nch, h->maxN, h->team, n - 1, spare, h->st);
     tmark(h, DQMC_PROF_STAB);
-    launch_green(h->d_chains, h->nch, spare, n, 0, 0, 0, 0, 0, h->st);
+    launch_green(h->d_chains, h->nch, h->maxN, h->team, spare, n, 0, h->st);
     tmark(h, DQMC_PROF_GREEN);
     launch_wrap_check(h->d_chains, h->nch, record, h->st);
     launch_swap_slots(h->d_slotmap, n, spare, h->st);
@@ -1624,9 +1624,9 @@ static void stab_b0(dqmc_handle* h, int n) {
     tmark(h, DQMC_PROF_OTHER);
     launch_bmat(h, 2, m.wrap_step[n * 2 + 1], m.wrap_step[n * 2], 1);
     tmark(h, DQMC_PROF_BPROD);
-    launch_stab_slots(h->d_chains, h->nch, n + 1, spare, h->st);
+    launch_stab_slots(h->d_chains, h->nch, h->maxN, h->team, n + 1, spare, h->st);
     tmark(h, DQMC_PROF_STAB);
-    launch_green(h->d_chains, h->nch, n, spare, 0, 0, 0, 0, 0, h->st);
+    launch_green(h->d_chains, h->nch, h->maxN, h->team, n, spare, 0, h->st);
     tmark(h, DQMC_PROF_GREEN);
     launch_wrap_check(h->d_chains, h->nch, 1, h->st);
     launch_swap_slots(h->d_slotmap, n, spare, h->st);
@@ -1700,7 +1700,7 @@ static void launch_measure_h(dqmc_handle* h) {
 
 // ULRINV = (UL UR)^-1 fresh, G = I - UR ULRINV UL, equaltime_measure
 static void proj_measure(dqmc_handle* h) {
-    launch_proj_ulr(h->d_chains, h->nch, PMAT_ULRINV, 0, 0, -1, h->st);
+    launch_proj_ulr(h->d_chains, h->nch, h->maxN, h->team, PMAT_ULRINV, 0, 0, -1, h->st);
     launch_proj_green(h->d_chains, h->nch, PMAT_ULRINV, PMAT_G, h->ctas_per_chain, h->st);
     tmark(h, DQMC_PROF_GREEN);
     launch_measure_h(h);
@@ -1709,7 +1709,7 @@ static void proj_measure(dqmc_handle* h) {
 
 // G of the current (UL, UR) into G, before a stabilisation replaces them
 static void proj_old_green(dqmc_handle* h) {
-    launch_proj_ulr(h->d_chains, h->nch, PMAT_W3, 0, 0, -1, h->st);
+    launch_proj_ulr(h->d_chains, h->nch, h->maxN, h->team, PMAT_W3, 0, 0, -1, h->st);
     launch_proj_green(h->d_chains, h->nch, PMAT_W3, PMAT_G, h->ctas_per_chain, h->st);
     tmark(h, DQMC_PROF_GREEN);
 }
@@ -1720,9 +1720,9 @@ static void stab_proj_0b(dqmc_handle* h, int n) {
     proj_old_green(h);
     launch_tall_copy(h->d_chains, h->nch, PMAT_ULT, PMAT_PST0 + n, h->st);
     tmark(h, DQMC_PROF_OTHER);
-    launch_proj_qr(h->d_chains, h->nch, PMAT_UR, n, n - 1, h->st);
+    launch_proj_qr(h->d_chains, h->nch, h->maxN, h->team, PMAT_UR, n, n - 1, h->st);
     tmark(h, DQMC_PROF_STAB);
-    launch_proj_ulr(h->d_chains, h->nch, PMAT_ULRINV, 1, n, n == nst ? -1 : n + 1, h->st);
+    launch_proj_ulr(h->d_chains, h->nch, h->maxN, h->team, PMAT_ULRINV, 1, n, n == nst ? -1 : n + 1, h->st);
     launch_proj_green(h->d_chains, h->nch, PMAT_ULRINV, PMAT_GNEW, h->ctas_per_chain, h->st);
     tmark(h, DQMC_PROF_GREEN);
     launch_wrap_check(h->d_chains, h->nch, 1, h->st);
@@ -1736,9 +1736,9 @@ static void stab_proj_b0(dqmc_handle* h, int n) {
     proj_old_green(h);
     launch_tall_copy(h->d_chains, h->nch, PMAT_UR, PMAT_PST0 + n, h->st);
     tmark(h, DQMC_PROF_OTHER);
-    launch_proj_qr(h->d_chains, h->nch, PMAT_ULT, n + 1, (n + 1 == nst) ? -1 : n + 2, h->st);
+    launch_proj_qr(h->d_chains, h->nch, h->maxN, h->team, PMAT_ULT, n + 1, (n + 1 == nst) ? -1 : n + 2, h->st);
     tmark(h, DQMC_PROF_STAB);
-    launch_proj_ulr(h->d_chains, h->nch, PMAT_ULRINV, 1, n + 1, n == 0 ? -1 : n, h->st);
+    launch_proj_ulr(h->d_chains, h->nch, h->maxN, h->team, PMAT_ULRINV, 1, n + 1, n == 0 ? -1 : n, h->st);
     launch_proj_green(h->d_chains, h->nch, PMAT_ULRINV, PMAT_GNEW, h->ctas_per_chain, h->st);
     tmark(h, DQMC_PROF_GREEN);
     launch_wrap_check(h->d_chains, h->nch, 1, h->st);
@@ -1773,11 +1773,11 @@ static int proj_sweep_start(dqmc_handle* h, int sync) {
         ProjPass pp;
         proj_bmat(h, pp, m.wrap_step[(n - 1) * 2 + 1], m.wrap_step[(n - 1) * 2]);
         pflush(h, pp);
-        launch_proj_qr(h->d_chains, h->nch, PMAT_UR, n, n - 1, h->st);
+        launch_proj_qr(h->d_chains, h->nch, h->maxN, h->team, PMAT_UR, n, n - 1, h->st);
         launch_tall_copy(h->d_chains, h->nch, PMAT_PST0 + n, PMAT_UR, h->st);
     }
     launch_tall_copy(h->d_chains, h->nch, PMAT_ULT, PMAT_PROJLC, h->st);
-    launch_proj_ulr(h->d_chains, h->nch, PMAT_ULRINV, 1, nst, -1, h->st);
+    launch_proj_ulr(h->d_chains, h->nch, h->maxN, h->team, PMAT_ULRINV, 1, nst, -1, h->st);
     launch_proj_green(h->d_chains, h->nch, PMAT_ULRINV, PMAT_GNEW, h->ctas_per_chain, h->st);
     launch_wrap_check(h->d_chains, h->nch, 0, h->st);
     if (sync) {
@@ -1866,7 +1866,7 @@ static void proj_dyn(dqmc_handle* h) {
         const int ntau = nt - t0;
         if (m.iwrap_nt[nt] > 0 || ntau == 0) {
             if (ntau > 0) launch_tall_copy(h->d_chains, h->nch, PMAT_ULT, PMAT_PST0 + m.iwrap_nt[nt], h->st);
-            launch_proj_ulr(h->d_chains, h->nch, PMAT_W3, 0, 0, -1, h->st);
+            launch_proj_ulr(h->d_chains, h->nch, h->maxN, h->team, PMAT_W3, 0, 0, -1, h->st);
             if (ntau == 0) {
                 launch_proj_green(h->d_chains, h->nch, PMAT_W3, PMAT_G, h->ctas_per_chain, h->st);
                 launch_dyn_init(h->d_chains, h->nch, h->st);
@@ -1888,7 +1888,7 @@ static void proj_dyn(dqmc_handle* h) {
         ProjPass pp;
         proj_bmat(h, pp, nt1, nt1);
         pflush(h, pp);
-        if (m.iwrap_nt[nt] > 0 && nt1 != t0 + ntdm) launch_proj_qr(h->d_chains, h->nch, PMAT_UR, -1, -1, h->st);
+        if (m.iwrap_nt[nt] > 0 && nt1 != t0 + ntdm) launch_proj_qr(h->d_chains, h->nch, h->maxN, h->team, PMAT_UR, -1, -1, h->st);
     }
     launch_tall_copy(h->d_chains, h->nch, PMAT_UR, PMAT_URS, h->st);
     launch_tall_copy(h->d_chains, h->nch, PMAT_ULT, PMAT_ULTS, h->st);
@@ -1953,9 +1953,9 @@ static int sweep_start_impl(dqmc_handle* h, int sync = 1) {
     for (int n = 1; n <= h->nst; ++n) {
         launch_copy_mat(h->d_chains, h->nch, 2, MAT_U + (n - 1), 0, h->st);
         launch_bmat(h, 2, m.wrap_step[(n - 1) * 2 + 1], m.wrap_step[(n - 1) * 2], 0);
-        launch_stab_slots(h->d_chains, h->nch, n - 1, n, h->st);
+        launch_stab_slots(h->d_chains, h->nch, h->maxN, h->team, n - 1, n, h->st);
     }
-    launch_green(h->d_chains, h->nch, h->nst, 0, 0, 0, 0, 0, 1, h->st);
+    launch_green(h->d_chains, h->nch, h->maxN, h->team, h->nst, 0, 1, h->st);
     launch_wrap_check(h->d_chains, h->nch, 0, h->st);
     if (sync) {
         CK(cudaStreamSynchronize(h->st));
@@ -2204,8 +2204,8 @@ static void stab_dyn(dqmc_handle* h, int n) {
     int spare = h->nst + 1;
     launch_copy_mat(h->d_chains, h->nch, 2 /*W0*/, MAT_U + (n - 1), 0, h->st);
     launch_bmat(h, 2, m.wrap_step[(n - 1) * 2 + 1], m.wrap_step[(n - 1) * 2], 0);
-    launch_stab_slots(h->d_chains, h->nch, n - 1, spare, h->st);
-    launch_green_tau(h->d_chains, h->nch, spare, n, h->st);
+    launch_stab_slots(h->d_chains, h->nch, h->maxN, h->team, n - 1, spare, h->st);
+    launch_green_tau(h->d_chains, h->nch, h->maxN, h->team, spare, n, h->st);
     launch_wrap_check(h->d_chains, h->nch, 1, h->st);
     launch_swap_slots(h->d_slotmap, n, spare, h->st);
 }
@@ -2600,7 +2600,7 @@ extern "C" int dqmc_gpu_test_zgemm(dqmc_handle* h, int m, int n, int k, int opa,
 extern "C" int dqmc_gpu_test_qr(dqmc_handle* h, int a, int q, double* logdetq) {
     if (!h) return fail(DQMC_EINVAL, "null handle");
     if (a < 0 || a > 4 || q < 0 || q > 4 || a == q) return fail(DQMC_EINVAL, "work index 0..4, a != q");
-    launch_qr_test(h->d_chains, h->nch, 2 + a, 2 + q, h->st);
+    launch_qr_test(h->d_chains, h->nch, h->maxN, h->team, 2 + a, 2 + q, h->st);
     CK(cudaStreamSynchronize(h->st));
     CK(cudaGetLastError());
     for (int c = 0; c < h->nch; ++c) {
@@ -2794,8 +2794,8 @@ extern "C" int dqmc_gpu_time_op(dqmc_handle* h, int op, int reps, double* ms_out
     auto enqueue = [&]() {
         switch (op) {
         case 0: launch_update(h->d_chains, h->nch, 1, 0, h->st); break;
-        case 1: launch_stab_slots(h->d_chains, h->nch, 0, spare, h->st); break;
-        case 2: launch_green(h->d_chains, h->nch, 1, 0, 0, 0, 0, 0, 0, h->st); break;
+        case 1: launch_stab_slots(h->d_chains, h->nch, h->maxN, h->team, 0, spare, h->st); break;
+        case 2: launch_green(h->d_chains, h->nch, h->maxN, h->team, 1, 0, 0, h->st); break;
         case 3: { PropProg p; p.n = 0; prog_k(m, p, PW_INV, 0); prog_v(m, p, PW_INV, 1); prog_k(m, p, PW_INV, 1);
                   launch_prog(h, MAT_G, p, 0); break; }
         case 4: launch_measure_h(h); break;
@@ -2811,8 +2811,8 @@ extern "C" int dqmc_gpu_time_op(dqmc_handle* h, int op, int reps, double* ms_out
     auto enqueue_proj = [&]() {
         switch (op) {
         case 0: proj_update(h, 1, pnf, 0, 0, -1); break;
-        case 1: launch_proj_qr(h->d_chains, h->nch, PMAT_UR, 1, 0, h->st); break;
-        case 2: launch_proj_ulr(h->d_chains, h->nch, PMAT_ULRINV, 1, 1, -1, h->st);
+        case 1: launch_proj_qr(h->d_chains, h->nch, h->maxN, h->team, PMAT_UR, 1, 0, h->st); break;
+        case 2: launch_proj_ulr(h->d_chains, h->nch, h->maxN, h->team, PMAT_ULRINV, 1, 1, -1, h->st);
                 launch_proj_green(h->d_chains, h->nch, PMAT_ULRINV, PMAT_GNEW, h->ctas_per_chain, h->st); break;
         case 3: case 5: {
             ProjPass pp;
@@ -3016,7 +3016,7 @@ extern "C" int dqmc_gpu_proj_green(dqmc_handle* h) {
     if (!h) return fail(DQMC_EINVAL, "null handle");
     if (!h->proj) return fail(DQMC_ESTATE, "not a projective handle (params.proj = 0)");
     clear_fail(h);
-    launch_proj_ulr(h->d_chains, h->nch, PMAT_ULRINV, 0, 0, -1, h->st);
+    launch_proj_ulr(h->d_chains, h->nch, h->maxN, h->team, PMAT_ULRINV, 0, 0, -1, h->st);
     launch_proj_green(h->d_chains, h->nch, PMAT_ULRINV, PMAT_G, h->ctas_per_chain, h->st);
     return finish_checked(h, 0);
 }

@@ -65,7 +65,8 @@ static size_t proj_la_smem(int maxN) {
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_proj_qr(const ChainDev* __restrict__ chains, int mat_id, int dst, int add) {
     extern __shared__ double2 ssm[];
-    const ChainDev c = chains[blockIdx.x];
+    const Team tm = this_team();
+    const ChainDev c = chains[blockIdx.x / tm.size];
     const ModelDev& md = *c.md;
     const int N = c.N, ne = md.ne, tid = threadIdx.x, nth = blockDim.x;
     double2* buf = ssm;
@@ -73,9 +74,12 @@ __global__ void __launch_bounds__(256) k_proj_qr(const ChainDev* __restrict__ ch
     LinalgScratch sc = proj_scratch(c);
     double2* X = chain_mat(c, mat_id);
     double2* A = c.W[1];
-    for (size_t e = tid; e < (size_t)N * ne; e += nth) A[e] = X[e];
-    __syncthreads();
-    cta_qr64(A, N, sc, buf, buf, &S->L, ne);
+    for (int e = tm.rank * nth + tid; e < N * ne; e += tm.size * nth) A[e] = X[e];
+    tm.sync();
+    cta_qr64(A, N, sc, buf, buf, &S->L, tm, ne);
+    cta_form_q64(N, X, sc, buf, tm, ne);
+    tm.sync();
+    if (tm.rank) return;
     double lg = 0.0, neg = 0.0;
     for (int i = tid; i < ne; i += nth) {
         double r = A[MIDX(i, i, N)].x;
@@ -84,8 +88,6 @@ __global__ void __launch_bounds__(256) k_proj_qr(const ChainDev* __restrict__ ch
     }
     lg = block_sum(lg, S->red);
     neg = block_sum(neg, S->red);
-    cta_form_q64(A, N, X, sc, buf, ne);
-    __syncthreads();
     if (((long long)llround(neg)) & 1)
         for (int i = tid; i < N; i += nth) X[i] = cmk(-X[i].x, -X[i].y);
     if (tid == 0 && dst >= 0) c.logwDV[dst] = (add >= 0 ? c.logwDV[add] : 0.0) + lg;
@@ -97,7 +99,8 @@ __global__ void __launch_bounds__(256) k_proj_qr(const ChainDev* __restrict__ ch
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_proj_ulr(const ChainDev* __restrict__ chains, int out_id, int logdet, int ia, int ib) {
     extern __shared__ double2 ssm[];
-    const ChainDev c = chains[blockIdx.x];
+    const Team tm = this_team();
+    const ChainDev c = chains[blockIdx.x / tm.size];
     const ModelDev& md = *c.md;
     const int N = c.N, ne = md.ne, tid = threadIdx.x, nth = blockDim.x;
     double2* buf = ssm;
@@ -107,18 +110,21 @@ __global__ void __launch_bounds__(256) k_proj_ulr(const ChainDev* __restrict__ c
     ZGemmArgs g;
     g.M = ne; g.N = ne; g.K = N; g.alpha = cmk(1, 0); g.beta = cmk(0, 0);
     g.A = c.ULT; g.lda = N; g.opA = OP_T; g.B = c.UR; g.ldb = N; g.opB = OP_N; g.C = M; g.ldc = ne;
-    zgemm_cta<GemmBig>(g, 0, 1, buf);
-    cta_qr64(M, ne, sc, buf, buf, &S->L);
+    team_zgemm(g, tm, buf);
+    tm.sync();
+    cta_qr64(M, ne, sc, buf, buf, &S->L, tm);
     double2 ld = cmk(0, 0);
     int bad = 0;
-    for (int i = tid; i < ne; i += nth) {
-        const double r = M[MIDX(i, i, ne)].x;
-        bad |= (r == 0.0 || !isfinite(r));
+    if (tm.rank == 0) {
+        for (int i = tid; i < ne; i += nth) {
+            const double r = M[MIDX(i, i, ne)].x;
+            bad |= (r == 0.0 || !isfinite(r));
+        }
+        // a zero or non-finite pivot of UL UR: zgetrf's info > 0 in s_inv_logdet_lu_z
+        bad = __syncthreads_or(bad);
+        if (bad && tid == 0) chain_raise(c, DQ_FAIL_SINGULAR);
     }
-    // a zero or non-finite pivot of UL UR: zgetrf's info > 0 in s_inv_logdet_lu_z
-    bad = __syncthreads_or(bad);
-    if (bad && tid == 0) chain_raise(c, DQ_FAIL_SINGULAR);
-    if (logdet) {
+    if (logdet && tm.rank == 0) {
         ld = cta_logdet_q(sc.tau, ne, S->red);
         double2 lr = cmk(0, 0);
         for (int i = tid; i < ne; i += nth) {
@@ -129,11 +135,15 @@ __global__ void __launch_bounds__(256) k_proj_ulr(const ChainDev* __restrict__ c
         ld = cadd(ld, lr);
     }
     double2* X = chain_mat(c, out_id);
-    for (int e = tid; e < ne * ne; e += nth) X[e] = cmk((e % ne) == (e / ne) ? 1.0 : 0.0, 0.0);
-    __syncthreads();
-    cta_apply_qh64(M, ne, X, sc, buf);
-    cta_trsm_upper(M, ne, X, buf, &S->L);
-    if (logdet && tid == 0) {
+    const int w = tm.chunk(ne);
+    for (int c0 = tm.rank * w; c0 < ne; c0 += tm.size * w) {
+        const int nc = min(w, ne - c0);
+        for (int e = tid; e < ne * nc; e += nth) X[e + c0 * ne] = cmk((e % ne) == c0 + e / ne ? 1.0 : 0.0, 0.0);
+        __syncthreads();
+        cta_apply_qh64(ne, X, c0, nc, sc, buf);
+        cta_trsm_upper64(M, ne, X, c0, nc, buf, &S->L);
+    }
+    if (logdet && tm.rank == 0 && tid == 0) {
         double w = c.logwDV[ia] + (ib >= 0 ? c.logwDV[ib] : 0.0);
         c.stats[ST_LOGDETM_RE] = ld.x + w;
         c.stats[ST_LOGDETM_IM] = ld.y;
@@ -494,15 +504,16 @@ __global__ void __launch_bounds__(256) k_pwin_seq(const ChainDev* __restrict__ c
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
+static constexpr size_t PUPD_SMEM = (size_t)ZT_SMEM_ELEMS * sizeof(double2) + sizeof(PUpdSmem) + 64;
 static int g_proj_attr = 0;
-static size_t g_proj_la = 0, g_proj_upd = 0;
 
-void set_proj_maxN(int maxN) {
-    g_proj_la = proj_la_smem(maxN);
-    g_proj_upd = (size_t)ZT_SMEM_ELEMS * sizeof(double2) + sizeof(PUpdSmem) + 64;
-    cudaFuncSetAttribute(k_proj_qr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g_proj_la);
-    cudaFuncSetAttribute(k_proj_ulr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g_proj_la);
-    cudaFuncSetAttribute(k_pwin_seq, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g_proj_upd);
+static void proj_attrs() {
+    if (g_proj_attr) return;
+    for (const void* k : {(const void*)k_proj_qr, (const void*)k_proj_ulr}) {
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, TEAM_SMEM_MAX);
+        cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    }
+    cudaFuncSetAttribute(k_pwin_seq, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PUPD_SMEM);
     cudaFuncSetAttribute(k_pwin_rg, cudaFuncAttributeMaxDynamicSharedMemorySize, ZT_SMEM_ELEMS * (int)sizeof(double2));
     cudaFuncSetAttribute(k_pwin_flush, cudaFuncAttributeMaxDynamicSharedMemorySize, ZT_SMEM_ELEMS * (int)sizeof(double2));
     cudaFuncSetAttribute(k_proj_t1, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmBig::SMEM_ELEMS * (int)sizeof(double2));
@@ -510,16 +521,19 @@ void set_proj_maxN(int maxN) {
     g_proj_attr = 1;
 }
 
-void launch_proj_qr(const ChainDev* chains, int nchains, int mat_id, int dst, int add, cudaStream_t st) {
-    k_proj_qr<<<nchains, 256, g_proj_la, st>>>(chains, mat_id, dst, add);
+void launch_proj_qr(const ChainDev* chains, int nchains, int maxN, int team, int mat_id, int dst, int add, cudaStream_t st) {
+    proj_attrs();
+    launch_team(k_proj_qr, nchains, team, proj_la_smem(maxN), st, chains, mat_id, dst, add);
 }
 
-void launch_proj_ulr(const ChainDev* chains, int nchains, int out_id, int logdet, int ia, int ib, cudaStream_t st) {
-    k_proj_ulr<<<nchains, 256, g_proj_la, st>>>(chains, out_id, logdet, ia, ib);
+void launch_proj_ulr(const ChainDev* chains, int nchains, int maxN, int team, int out_id, int logdet, int ia, int ib, cudaStream_t st) {
+    proj_attrs();
+    launch_team(k_proj_ulr, nchains, team, proj_la_smem(maxN), st, chains, out_id, logdet, ia, ib);
 }
 
 void launch_proj_green(const ChainDev* chains, int nchains, int inv_id, int dst_id, int ctas, cudaStream_t st) {
     size_t sm = (size_t)GemmBig::SMEM_ELEMS * sizeof(double2);
+    proj_attrs();
     k_proj_t1<<<dim3(ctas, nchains), 256, sm, st>>>(chains, inv_id);
     k_proj_gmat<<<dim3(ctas, nchains), 256, sm, st>>>(chains, dst_id);
 }
@@ -533,9 +547,10 @@ void launch_tall_copy(const ChainDev* chains, int nchains, int dst_id, int src_i
 void launch_proj_update(const ChainDev* chains, int nchains, int nt, int nf, int visit, int dir, int rnd_off,
                         int nwin, int g_rg, int g_fl, cudaStream_t st) {
     size_t sm = (size_t)ZT_SMEM_ELEMS * sizeof(double2);
+    proj_attrs();
     for (int w = 0; w < nwin; ++w) {
         k_pwin_rg<<<dim3(g_rg, nchains), 256, sm, st>>>(chains, nf, w);
-        k_pwin_seq<<<nchains, 256, g_proj_upd, st>>>(chains, nt, nf, w, visit, dir, rnd_off);
+        k_pwin_seq<<<nchains, 256, PUPD_SMEM, st>>>(chains, nt, nf, w, visit, dir, rnd_off);
         k_pwin_flush<<<dim3(g_fl, nchains), 256, sm, st>>>(chains, nf, w);
     }
 }

@@ -39,10 +39,24 @@ static size_t stab_smem_bytes(int maxN) {
     return (a > b ? a : b) * sizeof(double2) + sizeof(StabSmem) + 64;
 }
 
+// The chain of this CTA and its place in the chain's team (grid: nchains x team
+// size CTAs, a cluster per chain).
+DQ_DEV int team_chain(const Team& tm) { return blockIdx.x / tm.size; }
+
+// f(i, j) over the elements of an n x nc matrix, a column per warp, columns
+// dealt out over the team's warps
+template <class F>
+DQ_DEV void team_each(const Team& tm, int n, int nc, F f) {
+    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    for (int j = tm.rank * nw + (threadIdx.x >> 5); j < nc; j += tm.size * nw)
+        for (int i = lane; i < n; i += 32) f(i, j);
+}
+
 // one UDV step: W0 holds B(slices) * U[src]; writes U/D/V/logdetQ of slot dst.
 __global__ void __launch_bounds__(256, 2) k_stab(const ChainDev* __restrict__ chains, int src, int dst) {
     extern __shared__ double2 ssm[];
-    const ChainDev c = chains[blockIdx.x];
+    const Team tm = this_team();
+    const ChainDev c = chains[team_chain(tm)];
     const int N = c.N, tid = threadIdx.x, nth = blockDim.x;
     const size_t NN = (size_t)N * N;
     double2* buf = ssm;
@@ -61,15 +75,15 @@ __global__ void __launch_bounds__(256, 2) k_stab(const ChainDev* __restrict__ ch
 
     // column norms of B U D (s_z_x_diag_d + s_zmcpt)
     const int lane = tid & 31, warp = tid >> 5, nw = nth >> 5;
-    for (int j = warp; j < N; j += nw) {
+    for (int j = tm.rank * nw + warp; j < N; j += tm.size * nw) {
         double s = 0.0;
         for (int r = lane; r < N; r += 32) s += cabs2(W0[MIDX(r, j, N)]);
         s = warp_sum(s);
         if (lane == 0) nrm[j] = sqrt(s) * fabs(Dsrc[j]);
     }
-    __syncthreads();
+    tm.sync();
     // descending stable rank sort
-    for (int j = tid; j < N; j += nth) {
+    for (int j = tm.rank * nth + tid; j < N; j += tm.size * nth) {
         double v = nrm[j];
         int rank = 0;
         for (int k = 0; k < N; ++k) {
@@ -78,44 +92,40 @@ __global__ void __launch_bounds__(256, 2) k_stab(const ChainDev* __restrict__ ch
         }
         perm[rank] = j;
     }
-    __syncthreads();
-    for (size_t e = tid; e < NN; e += nth) {
-        int r = (int)(e % N), k = (int)(e / N);
-        int j = perm[k];
-        W2[e] = cscale(W0[MIDX(r, j, N)], Dsrc[j]);
-    }
-    __syncthreads();
-    cta_qr64(W2, N, sc, buf, buf, &S->L);
-    int bad = 0;
-    for (int i = tid; i < N; i += nth) {
-        const double d = W2[MIDX(i, i, N)].x;
-        Ddst[i] = d;
-        bad |= (d == 0.0 || !isfinite(d));
-    }
-    // a zero or non-finite R_ii (the zgeqp3 / zgeqrf step of the reference)
-    if (__syncthreads_or(bad) && tid == 0) chain_raise(c, DQ_FAIL_SINGULAR);
-    double2 ldq = cta_logdet_q(sc.tau, N, S->red);
-    if (tid == 0) c.logdetQ[dst] = ldq;
-    __syncthreads();
-    // Vt = D^-1 R
-    for (size_t e = tid; e < NN; e += nth) {
-        int r = (int)(e % N), k = (int)(e / N);
-        W3[e] = (r <= k) ? cscale(W2[e], 1.0 / Ddst[r]) : cmk(0, 0);
-    }
+    tm.sync();
+    team_each(tm, N, N, [&](int r, int k) {
+        const int j = perm[k];
+        W2[MIDX(r, k, N)] = cscale(W0[MIDX(r, j, N)], Dsrc[j]);
+    });
     // P^T V_src: row k <- row perm[k]
     const double2* Vsrc = c.V + (size_t)src * NN;
-    for (size_t e = tid; e < NN; e += nth) {
-        int r = (int)(e % N), k = (int)(e / N);
-        W4[e] = Vsrc[MIDX(perm[r], k, N)];
+    team_each(tm, N, N, [&](int r, int k) { W4[MIDX(r, k, N)] = Vsrc[MIDX(perm[r], k, N)]; });
+    tm.sync();
+    cta_qr64(W2, N, sc, buf, buf, &S->L, tm);
+    if (tm.rank == 0) {
+        int bad = 0;
+        for (int i = tid; i < N; i += nth) {
+            const double d = W2[MIDX(i, i, N)].x;
+            Ddst[i] = d;
+            bad |= (d == 0.0 || !isfinite(d));
+        }
+        // a zero or non-finite R_ii (the zgeqp3 / zgeqrf step of the reference)
+        if (__syncthreads_or(bad) && tid == 0) chain_raise(c, DQ_FAIL_SINGULAR);
+        double2 ldq = cta_logdet_q(sc.tau, N, S->red);
+        if (tid == 0) c.logdetQ[dst] = ldq;
     }
-    __syncthreads();
-    cta_form_q64(W2, N, c.U + (size_t)dst * NN, sc, buf);
+    // Vt = D^-1 R
+    team_each(tm, N, N, [&](int r, int k) {
+        W3[MIDX(r, k, N)] = (r <= k) ? cscale(W2[MIDX(r, k, N)], 1.0 / W2[MIDX(r, r, N)].x) : cmk(0, 0);
+    });
+    cta_form_q64(N, c.U + (size_t)dst * NN, sc, buf, tm);
+    tm.sync();
     ZGemmArgs g;
     g.M = N; g.N = N; g.K = N; g.alpha = cmk(1, 0); g.beta = cmk(0, 0);
     g.A = W3; g.lda = N; g.opA = OP_N; g.B = W4; g.ldb = N; g.opB = OP_N;
     g.C = c.V + (size_t)dst * NN; g.ldc = N;
     g.triA = 1;                          // D^-1 R is upper triangular
-    zgemm_cta<GemmBig>(g, 0, 1, buf);
+    team_zgemm(g, tm, buf);
 }
 
 // s_dvec_min_max
@@ -124,11 +134,29 @@ DQ_DEV void dminmax(double d, double& dmax, double& dmin) {
     else { dmax = 1.0; dmin = d; }
 }
 
+// X(:, c0:c0+nc) = diag(s)^-1 (U^H)(:, c0:c0+nc), 32 x 32 tiles through shared memory
+// (buf holds 32 x 33 elements); one CTA
+DQ_DEV void cta_conj_transpose(const double2* U, int N, double2* X, int c0, int nc, const double* s, double2* buf) {
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (int j0 = 0; j0 < nc; j0 += 32)
+        for (int i0 = 0; i0 < N; i0 += 32) {
+            const int r = c0 + j0 + tx;              // rows of U are columns of X
+            for (int k = ty; k < 32; k += nw)
+                if (j0 + tx < nc && i0 + k < N) buf[k * 33 + tx] = U[MIDX(r, i0 + k, N)];
+            __syncthreads();
+            for (int k = ty; k < 32; k += nw)
+                if (i0 + tx < N && j0 + k < nc)
+                    X[MIDX(i0 + tx, c0 + j0 + k, N)] = cscale(cconj(buf[tx * 33 + k]), 1.0 / s[i0 + tx]);
+            __syncthreads();
+        }
+}
+
 // Green's function into Gnew.  mode 0: green_equaltime(R = slot nr, L = slot nl);
 // mode 1: green_equaltimebb (R = slot nr).  New log weight -> stats[ST_LOGDETM_*].
 __global__ void __launch_bounds__(256, 2) k_green(const ChainDev* __restrict__ chains, int nr, int nl, int mode) {
     extern __shared__ double2 ssm[];
-    const ChainDev c = chains[blockIdx.x];
+    const Team tm = this_team();
+    const ChainDev c = chains[team_chain(tm)];
     const int N = c.N, tid = threadIdx.x, nth = blockDim.x;
     const size_t NN = (size_t)N * N;
     double2* buf = ssm;
@@ -139,6 +167,9 @@ __global__ void __launch_bounds__(256, 2) k_green(const ChainDev* __restrict__ c
     const double2* UR = c.U + (size_t)nr * NN;
     const double2* VR = c.V + (size_t)nr * NN;
     const double* DR = c.D + (size_t)nr * N;
+    const double2* UL = c.U + (size_t)nl * NN;       // mode 0 only
+    const double2* VL = c.V + (size_t)nl * NN;
+    const double* DL = c.D + (size_t)nl * N;
     double* drmax = c.vecs + 0 * N;
     double* drmin = c.vecs + 1 * N;
     double* dlmax = c.vecs + 2 * N;
@@ -146,78 +177,75 @@ __global__ void __launch_bounds__(256, 2) k_green(const ChainDev* __restrict__ c
     double2* M = c.W[0];
     double2* Z = c.W[1];
     double slog = 0.0;
-    for (int i = tid; i < N; i += nth) {
-        double a, b;
-        dminmax(DR[i], a, b);
-        drmax[i] = a; drmin[i] = b;
-        slog += log(a);
-    }
-    if (mode == 0) {
-        const double2* UL = c.U + (size_t)nl * NN;
-        const double2* VL = c.V + (size_t)nl * NN;
-        const double* DL = c.D + (size_t)nl * N;
+    if (tm.rank == 0)
         for (int i = tid; i < N; i += nth) {
             double a, b;
-            dminmax(DL[i], a, b);
-            dlmax[i] = a; dlmin[i] = b;
+            dminmax(DR[i], a, b);
+            drmax[i] = a; drmin[i] = b;
             slog += log(a);
+            if (mode == 0) {
+                dminmax(DL[i], a, b);
+                dlmax[i] = a; dlmin[i] = b;
+                slog += log(a);
+            }
         }
-        __syncthreads();   // dmax/dmin are read by other threads below
+    tm.sync();   // dmax/dmin are read by other threads below
+    if (mode == 0) {
         ZGemmArgs g;
         g.M = N; g.N = N; g.K = N; g.alpha = cmk(1, 0); g.beta = cmk(0, 0);
         g.A = UR; g.lda = N; g.opA = OP_C; g.B = UL; g.ldb = N; g.opB = OP_N; g.C = M; g.ldc = N;
-        zgemm_cta<GemmBig>(g, 0, 1, buf);
+        team_zgemm(g, tm, buf);
         g.A = VR; g.opA = OP_N; g.B = VL; g.opB = OP_C; g.C = Z;
-        zgemm_cta<GemmBig>(g, 0, 1, buf);
-        for (size_t e = tid; e < NN; e += nth) {
-            int i = (int)(e % N), j = (int)(e / N);
+        team_zgemm(g, tm, buf);
+        tm.sync();
+        team_each(tm, N, N, [&](int i, int j) {
+            const size_t e = MIDX(i, j, N);
             double2 u = cscale(M[e], 1.0 / (drmax[i] * dlmax[j]));
             M[e] = cadd(u, cscale(Z[e], drmin[i] * dlmin[j]));
-        }
+        });
     } else {
-        __syncthreads();   // drmax/drmin are read by other threads below
-        for (size_t e = tid; e < NN; e += nth) {
-            int i = (int)(e % N), j = (int)(e / N);
-            M[e] = cadd(cscale(cconj(UR[MIDX(j, i, N)]), 1.0 / drmax[i]), cscale(VR[e], drmin[i]));
-        }
+        team_each(tm, N, N, [&](int i, int j) {
+            M[MIDX(i, j, N)] = cadd(cscale(cconj(UR[MIDX(j, i, N)]), 1.0 / drmax[i]), cscale(VR[MIDX(i, j, N)], drmin[i]));
+        });
     }
-    slog = block_sum(slog, S->red);
-    __syncthreads();
-    cta_qr64(M, N, sc, buf, buf, &S->L);
-    double2 ldm = cta_logdet_q(sc.tau, N, S->red);
-    double2 lr = cmk(0, 0);
+    tm.sync();
+    cta_qr64(M, N, sc, buf, buf, &S->L, tm);
+    double2 ldm = cmk(0, 0);
     int bad = 0;
-    for (int i = tid; i < N; i += nth) {
-        double r = M[MIDX(i, i, N)].x;
-        bad |= (r == 0.0 || !isfinite(r));
-        lr = cadd(lr, cmk(log(fabs(r)), r < 0.0 ? M_PI : 0.0));
-    }
-    // a zero or non-finite pivot of M: zgetrf's info > 0 in s_inv_logdet_lu_z
-    bad = __syncthreads_or(bad);
-    lr = block_csum(lr, S->red);
-    ldm = cadd(ldm, lr);
-    double2* X = (mode == 0) ? Z : c.Gnew;
-    for (size_t e = tid; e < NN; e += nth) {
-        int i = (int)(e % N), j = (int)(e / N);
-        X[e] = cscale(cconj(UR[MIDX(j, i, N)]), 1.0 / drmax[i]);
-    }
-    __syncthreads();
-    cta_apply_qh64(M, N, X, sc, buf);
-    cta_trsm_upper64(M, N, X, buf, &S->L);
-    if (mode == 0) {
-        const double2* UL = c.U + (size_t)nl * NN;
-        double2* UL2 = c.W[2];
-        for (size_t e = tid; e < NN; e += nth) {
-            int j = (int)(e / N);
-            UL2[e] = cscale(UL[e], 1.0 / dlmax[j]);
+    if (tm.rank == 0) {
+        slog = block_sum(slog, S->red);
+        ldm = cta_logdet_q(sc.tau, N, S->red);
+        double2 lr = cmk(0, 0);
+        for (int i = tid; i < N; i += nth) {
+            double r = M[MIDX(i, i, N)].x;
+            bad |= (r == 0.0 || !isfinite(r));
+            lr = cadd(lr, cmk(log(fabs(r)), r < 0.0 ? M_PI : 0.0));
         }
+        // a zero or non-finite pivot of M: zgetrf's info > 0 in s_inv_logdet_lu_z
+        bad = __syncthreads_or(bad);
+        lr = block_csum(lr, S->red);
+        ldm = cadd(ldm, lr);
         __syncthreads();
+    }
+    // UL dlmax^-1, and X = M^-1 drmax^-1 UR^H by column chunks
+    double2* UL2 = c.W[2];
+    if (mode == 0) team_each(tm, N, N, [&](int i, int j) { UL2[MIDX(i, j, N)] = cscale(UL[MIDX(i, j, N)], 1.0 / dlmax[j]); });
+    double2* X = (mode == 0) ? Z : c.Gnew;
+    const int w = tm.chunk(N);
+    for (int c0 = tm.rank * w; c0 < N; c0 += tm.size * w) {
+        const int nc = min(w, N - c0);
+        cta_conj_transpose(UR, N, X, c0, nc, drmax, buf);
+        cta_apply_qh64(N, X, c0, nc, sc, buf);
+        cta_trsm_upper64(M, N, X, c0, nc, buf, &S->L);
+    }
+    if (mode == 0) {
+        tm.sync();
         ZGemmArgs g;
         g.M = N; g.N = N; g.K = N; g.alpha = cmk(1, 0); g.beta = cmk(0, 0);
         g.A = UL2; g.lda = N; g.opA = OP_N; g.B = Z; g.ldb = N; g.opB = OP_N; g.C = c.Gnew; g.ldc = N;
-        zgemm_cta<GemmBig>(g, 0, 1, buf);
+        team_zgemm(g, tm, buf);
     }
-    if (tid == 0) {
+    if (tm.rank == 0 && tid == 0) {
         double2 lw = cadd(ldm, cmk(slog, 0.0));
         lw = cadd(lw, c.logdetQ[nr]);
         if (mode == 0) lw = csub(lw, c.logdetQ[nl]);
@@ -242,7 +270,8 @@ __global__ void __launch_bounds__(256, 2) k_green(const ChainDev* __restrict__ c
 // the reflector blocks of the QR).
 __global__ void __launch_bounds__(256, 2) k_green_tau(const ChainDev* __restrict__ chains, int nr, int nl) {
     extern __shared__ double2 ssm[];
-    const ChainDev& c = chains[blockIdx.x];
+    const Team tm = this_team();
+    const ChainDev& c = chains[team_chain(tm)];
     const int N = c.N, tid = threadIdx.x, nth = blockDim.x;
     const size_t NN = (size_t)N * N;
     double2* buf = ssm;
@@ -262,97 +291,101 @@ __global__ void __launch_bounds__(256, 2) k_green_tau(const ChainDev* __restrict
     double* dlmin = c.vecs + 3 * N;
     double2 *W0 = c.W[0], *W1 = c.W[1], *W2 = c.W[2], *W3 = c.W[3], *W4 = c.W[4];
     double slog = 0.0;
-    for (int i = tid; i < N; i += nth) {
-        double a, b;
-        dminmax(DR[i], a, b);
-        drmax[i] = a; drmin[i] = b;
-        slog += log(a);
-        dminmax(DL[i], a, b);
-        dlmax[i] = a; dlmin[i] = b;
-        slog += log(a);
-    }
-    __syncthreads();
+    if (tm.rank == 0)
+        for (int i = tid; i < N; i += nth) {
+            double a, b;
+            dminmax(DR[i], a, b);
+            drmax[i] = a; drmin[i] = b;
+            slog += log(a);
+            dminmax(DL[i], a, b);
+            dlmax[i] = a; dlmin[i] = b;
+            slog += log(a);
+        }
+    tm.sync();
     ZGemmArgs g;
     g.M = N; g.N = N; g.K = N; g.alpha = cmk(1, 0); g.beta = cmk(0, 0); g.lda = N; g.ldb = N; g.ldc = N;
     auto gemm = [&](const double2* A, int opA, const double2* B, int opB, double2* C, double alpha) {
         g.A = A; g.opA = opA; g.B = B; g.opB = opB; g.C = C; g.alpha = cmk(alpha, 0);
-        zgemm_cta<GemmBig>(g, 0, 1, buf);
+        team_zgemm(g, tm, buf);
     };
     // uu = UR^H UL (W1, kept for M2), vv = VR VL^H (W2)
     gemm(UR, OP_C, UL, OP_N, W1, 1.0);
     gemm(VR, OP_N, VL, OP_C, W2, 1.0);
-    for (size_t e = tid; e < NN; e += nth) {
-        const int i = (int)(e % N), j = (int)(e / N);
+    tm.sync();
+    team_each(tm, N, N, [&](int i, int j) {
+        const size_t e = MIDX(i, j, N);
         W0[e] = cadd(cscale(W1[e], 1.0 / (drmax[i] * dlmax[j])), cscale(W2[e], drmin[i] * dlmin[j]));
-    }
-    slog = block_sum(slog, S->red);
-    __syncthreads();
-    cta_qr64(W0, N, sc, buf, buf, &S->L);
-    double2 ldm = cta_logdet_q(sc.tau, N, S->red);
-    double2 lr = cmk(0, 0);
+    });
+    tm.sync();
+    cta_qr64(W0, N, sc, buf, buf, &S->L, tm);
+    double2 ldm = cmk(0, 0);
     int bad = 0;
-    for (int i = tid; i < N; i += nth) {
-        const double r = W0[MIDX(i, i, N)].x;
-        bad |= (r == 0.0 || !isfinite(r));
-        lr = cadd(lr, cmk(log(fabs(r)), r < 0.0 ? M_PI : 0.0));
+    if (tm.rank == 0) {
+        slog = block_sum(slog, S->red);
+        ldm = cta_logdet_q(sc.tau, N, S->red);
+        double2 lr = cmk(0, 0);
+        for (int i = tid; i < N; i += nth) {
+            const double r = W0[MIDX(i, i, N)].x;
+            bad |= (r == 0.0 || !isfinite(r));
+            lr = cadd(lr, cmk(log(fabs(r)), r < 0.0 ? M_PI : 0.0));
+        }
+        bad = __syncthreads_or(bad);
+        lr = block_csum(lr, S->red);
+        ldm = cadd(ldm, lr);
+        __syncthreads();
     }
-    bad = __syncthreads_or(bad);
-    lr = block_csum(lr, S->red);
-    ldm = cadd(ldm, lr);
-    // X = M^-1 drmax^-1 UR^H (W2), Y = M^-1 drmin VR (W3)
-    for (size_t e = tid; e < NN; e += nth) {
-        const int i = (int)(e % N), j = (int)(e / N);
+    // X = M^-1 drmax^-1 UR^H (W2), Y = M^-1 drmin VR (W3), UL dlmax^-1 (W4)
+    team_each(tm, N, N, [&](int i, int j) {
+        const size_t e = MIDX(i, j, N);
         W2[e] = cscale(cconj(UR[MIDX(j, i, N)]), 1.0 / drmax[i]);
         W3[e] = cscale(VR[e], drmin[i]);
-    }
-    __syncthreads();
-    cta_apply_qh64(W0, N, W2, sc, buf);
-    cta_trsm_upper64(W0, N, W2, buf, &S->L);
-    cta_apply_qh64(W0, N, W3, sc, buf);
-    cta_trsm_upper64(W0, N, W3, buf, &S->L);
-    // UL dlmax^-1 (W4); G(tau,tau) and G(tau,0)
-    for (size_t e = tid; e < NN; e += nth) W4[e] = cscale(UL[e], 1.0 / dlmax[(int)(e / N)]);
-    __syncthreads();
+        W4[e] = cscale(UL[e], 1.0 / dlmax[j]);
+    });
+    tm.sync();
+    cta_solve64(W0, N, W2, sc, buf, &S->L, tm);
+    cta_solve64(W0, N, W3, sc, buf, &S->L, tm);
+    tm.sync();
+    // G(tau,tau) and G(tau,0)
     gemm(W4, OP_N, W2, OP_N, c.Gnew, 1.0);
     gemm(W4, OP_N, W3, OP_N, c.gt0, 1.0);
+    tm.sync();
     // VR^-1 (W2) and (VL^H)^-1 (W3) through QR: W0 <- A, W <- I, solve
     for (int pass = 0; pass < 2; ++pass) {
         double2* Xi = pass == 0 ? W2 : W3;
-        for (size_t e = tid; e < NN; e += nth) {
-            const int i = (int)(e % N), j = (int)(e / N);
+        team_each(tm, N, N, [&](int i, int j) {
+            const size_t e = MIDX(i, j, N);
             W0[e] = pass == 0 ? VR[e] : cconj(VL[MIDX(j, i, N)]);
             Xi[e] = cmk(i == j ? 1.0 : 0.0, 0.0);
-        }
-        __syncthreads();
-        cta_qr64(W0, N, sc, buf, buf, &S->L);
-        cta_apply_qh64(W0, N, Xi, sc, buf);
-        cta_trsm_upper64(W0, N, Xi, buf, &S->L);
+        });
+        tm.sync();
+        cta_qr64(W0, N, sc, buf, buf, &S->L, tm);
+        cta_solve64(W0, N, Xi, sc, buf, &S->L, tm);
+        tm.sync();
     }
     // (VR VL^H)^-1 = (VL^H)^-1 VR^-1 (W4); M2 (W0)
     gemm(W3, OP_N, W2, OP_N, W4, 1.0);
-    for (size_t e = tid; e < NN; e += nth) {
-        const int i = (int)(e % N), j = (int)(e / N);
+    tm.sync();
+    team_each(tm, N, N, [&](int i, int j) {
+        const size_t e = MIDX(i, j, N);
         W0[e] = cadd(cscale(W4[e], 1.0 / (dlmax[i] * drmax[j])), cscale(cconj(W1[MIDX(j, i, N)]), dlmin[i] * drmin[j]));
-    }
-    __syncthreads();
-    cta_qr64(W0, N, sc, buf, buf, &S->L);
-    // Z = M2^-1 dlmax^-1 (VL^H)^-1 (W3), Wm = M2^-1 (-dlmin UL^H) (W4)
-    for (size_t e = tid; e < NN; e += nth) {
-        const int i = (int)(e % N), j = (int)(e / N);
+    });
+    tm.sync();
+    cta_qr64(W0, N, sc, buf, buf, &S->L, tm);
+    // Z = M2^-1 dlmax^-1 (VL^H)^-1 (W3), Wm = M2^-1 (-dlmin UL^H) (W4), VR^-1 drmax^-1 (W2)
+    team_each(tm, N, N, [&](int i, int j) {
+        const size_t e = MIDX(i, j, N);
         W3[e] = cscale(W3[e], 1.0 / dlmax[i]);
         W4[e] = cscale(cconj(UL[MIDX(j, i, N)]), -dlmin[i]);
-    }
-    __syncthreads();
-    cta_apply_qh64(W0, N, W3, sc, buf);
-    cta_trsm_upper64(W0, N, W3, buf, &S->L);
-    cta_apply_qh64(W0, N, W4, sc, buf);
-    cta_trsm_upper64(W0, N, W4, buf, &S->L);
-    // VR^-1 drmax^-1 (W2); G(0,0), G(0,tau)
-    for (size_t e = tid; e < NN; e += nth) W2[e] = cscale(W2[e], 1.0 / drmax[(int)(e / N)]);
-    __syncthreads();
+        W2[e] = cscale(W2[e], 1.0 / drmax[j]);
+    });
+    tm.sync();
+    cta_solve64(W0, N, W3, sc, buf, &S->L, tm);
+    cta_solve64(W0, N, W4, sc, buf, &S->L, tm);
+    tm.sync();
+    // G(0,0), G(0,tau)
     gemm(W2, OP_N, W3, OP_N, c.g00, 1.0);
     gemm(W2, OP_N, W4, OP_N, c.g0t, 1.0);
-    if (tid == 0) {
+    if (tm.rank == 0 && tid == 0) {
         double2 lw = cadd(ldm, cmk(slog, 0.0));
         lw = cadd(lw, c.logdetQ[nr]);
         lw = csub(lw, c.logdetQ[nl]);
@@ -509,16 +542,19 @@ __global__ void __launch_bounds__(256) k_zgemm_test(const ChainDev* __restrict__
 // QR of matrix a_id in place; Q into q_id; logdetQ into stats[ST_LOGDETM]
 __global__ void __launch_bounds__(256) k_qr_test(const ChainDev* __restrict__ chains, int a_id, int q_id) {
     extern __shared__ double2 ssm[];
-    const ChainDev c = chains[blockIdx.x];
+    const Team tm = this_team();
+    const ChainDev c = chains[team_chain(tm)];
     const int N = c.N;
     StabSmem* S = (StabSmem*)(ssm + ((QR_PANEL_ELEMS(N) > (size_t)GemmBig::SMEM_ELEMS) ? QR_PANEL_ELEMS(N) : (size_t)GemmBig::SMEM_ELEMS));
     LinalgScratch sc = make_scratch(c);
     double2* A = chain_mat(c, a_id);
-    cta_qr64(A, N, sc, ssm, ssm, &S->L);
-    double2 ld = cta_logdet_q(sc.tau, N, S->red);
-    if (threadIdx.x == 0) { c.stats[ST_LOGDETM_RE] = ld.x; c.stats[ST_LOGDETM_IM] = ld.y; }
-    __syncthreads();
-    cta_form_q64(A, N, chain_mat(c, q_id), sc, ssm);
+    cta_qr64(A, N, sc, ssm, ssm, &S->L, tm);
+    if (tm.rank == 0) {
+        double2 ld = cta_logdet_q(sc.tau, N, S->red);
+        if (threadIdx.x == 0) { c.stats[ST_LOGDETM_RE] = ld.x; c.stats[ST_LOGDETM_IM] = ld.y; }
+        __syncthreads();
+    }
+    cta_form_q64(N, chain_mat(c, q_id), sc, ssm, tm);
 }
 
 // swap logical slot n with the spare slot (logical id `spare`)
@@ -531,39 +567,46 @@ __global__ void k_swap_slots(int* slotmap, int n, int spare) {
 static int g_stab_attr = 0;
 static void stab_attrs() {
     if (g_stab_attr) return;
-    cudaFuncSetAttribute(k_stab, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(k_green, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(k_green_tau, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(k_qr_test, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    for (const void* k : {(const void*)k_stab, (const void*)k_green, (const void*)k_green_tau, (const void*)k_qr_test}) {
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, TEAM_SMEM_MAX);
+        cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    }
     cudaFuncSetAttribute(k_zgemm_test, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     g_stab_attr = 1;
 }
 
-static int g_maxN = 512;
-void set_stab_maxN(int n) { g_maxN = n; }
-
-void launch_stab(const ChainDev* chains, int nchains, int n, int dir, int pivoted, cudaStream_t st) {
-    (void)pivoted;
+// CTAs per chain of the QR and Green's function kernels: the largest cluster of
+// which every chain gets one on SMs of its own.  A cluster lies inside one GPC, so
+// how many of a size fit is asked of the driver, for a block that fills an SM's
+// shared memory.  A second CTA on an SM does not pay: k_stab + k_green of 256
+// sites take 4.4 ms for 8 chains with 8 CTAs each and 5.2 ms with 16, and 5.4 ms
+// for 16 chains with 4 against 5.9 ms with 8 (10.8 ms with one CTA per chain).
+int pick_team(int nchains) {
     stab_attrs();
-    int src = dir == 0 ? n - 1 : n, dst = dir == 0 ? n : n - 1;
-    k_stab<<<nchains, 256, stab_smem_bytes(g_maxN), st>>>(chains, src, dst);
+    for (int t = 16; t > 1; t /= 2) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute at[1];
+        team_config(cfg, at, 1, t, TEAM_SMEM_MAX, 0);
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, k_green, &cfg) != cudaSuccess) { cudaGetLastError(); continue; }
+        if (nchains <= n) return t;
+    }
+    return 1;
 }
 
-void launch_stab_slots(const ChainDev* chains, int nchains, int src, int dst, cudaStream_t st) {
+void launch_stab_slots(const ChainDev* chains, int nchains, int maxN, int team, int src, int dst, cudaStream_t st) {
     stab_attrs();
-    k_stab<<<nchains, 256, stab_smem_bytes(g_maxN), st>>>(chains, src, dst);
+    launch_team(k_stab, nchains, team, stab_smem_bytes(maxN), st, chains, src, dst);
 }
 
-void launch_green(const ChainDev* chains, int nchains, int nr, int nl, int rmat_u, int rmat_v,
-                  int lmat_u, int lmat_v, int mode, cudaStream_t st) {
-    (void)rmat_u; (void)rmat_v; (void)lmat_u; (void)lmat_v;
+void launch_green(const ChainDev* chains, int nchains, int maxN, int team, int nr, int nl, int mode, cudaStream_t st) {
     stab_attrs();
-    k_green<<<nchains, 256, stab_smem_bytes(g_maxN), st>>>(chains, nr, nl, mode);
+    launch_team(k_green, nchains, team, stab_smem_bytes(maxN), st, chains, nr, nl, mode);
 }
 
-void launch_green_tau(const ChainDev* chains, int nchains, int nr, int nl, cudaStream_t st) {
+void launch_green_tau(const ChainDev* chains, int nchains, int maxN, int team, int nr, int nl, cudaStream_t st) {
     stab_attrs();
-    k_green_tau<<<nchains, 256, stab_smem_bytes(g_maxN), st>>>(chains, nr, nl);
+    launch_team(k_green_tau, nchains, team, stab_smem_bytes(maxN), st, chains, nr, nl);
 }
 
 void launch_stage(const ChainDev* chains, int nchains, int nslots, int dir, cudaStream_t st) {
@@ -703,7 +746,7 @@ void launch_zgemm_test(const ChainDev* chains, int nchains, int m, int n, int k,
     k_zgemm_test<<<grid, 256, GemmBig::SMEM_ELEMS * sizeof(double2), st>>>(chains, m, n, k, opa, opb, a_id, b_id, c_id, beta_re);
 }
 
-void launch_qr_test(const ChainDev* chains, int nchains, int a_id, int q_id, cudaStream_t st) {
+void launch_qr_test(const ChainDev* chains, int nchains, int maxN, int team, int a_id, int q_id, cudaStream_t st) {
     stab_attrs();
-    k_qr_test<<<nchains, 256, stab_smem_bytes(g_maxN), st>>>(chains, a_id, q_id);
+    launch_team(k_qr_test, nchains, team, stab_smem_bytes(maxN), st, chains, a_id, q_id);
 }

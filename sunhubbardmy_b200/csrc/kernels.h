@@ -38,21 +38,20 @@ void launch_update_flush(const ChainDev* chains, int nchains, cudaStream_t st); 
 enum { MEAS_ONE_ORBITAL = 0, MEAS_HONEYCOMB = 1, MEAS_CUBIC = 2, MEAS_R_CUBIC = 3 };
 void launch_measure(const ChainDev* chains, int nchains, int maxN, int kind, int maxlq, cudaStream_t st);
 void launch_bins_clear(const ChainDev* chains, int nchains, int nbins, cudaStream_t st);
-void launch_stab_slots(const ChainDev* chains, int nchains, int src, int dst, cudaStream_t st);
+// CTAs per chain (a thread-block cluster) of the stabilisation and Green's
+// function kernels of a handle of nchains chains
+int pick_team(int nchains);
+// UDV step: W0 = B(slices) U[src], the new factors into slot dst
+void launch_stab_slots(const ChainDev* chains, int nchains, int maxN, int team, int src, int dst, cudaStream_t st);
 void launch_swap_slots(int* slotmap, int n, int spare, cudaStream_t st);
 void launch_stack_identity(const ChainDev* chains, int nchains, int slot, cudaStream_t st);
-void set_stab_maxN(int n);
 void launch_copy_mat(const ChainDev* chains, int nchains, int dst_id, int src_id, int identity, cudaStream_t st);
-// stabilisation step: dir 0 = 0b (writes stack n from n-1), 1 = b0 (writes n-1 from n);
-// pivoted selects the QR with column pivoting of the first/last step.
-void launch_stab(const ChainDev* chains, int nchains, int n, int dir, int pivoted, cudaStream_t st);
 // Green's function from the stack entries (r side, l side) into Gnew; mode 0 =
 // green_equaltime, 1 = green_equaltimebb (l side = identity)
-void launch_green(const ChainDev* chains, int nchains, int nr, int nl, int rmat_u, int rmat_v,
-                  int lmat_u, int lmat_v, int mode, cudaStream_t st);
+void launch_green(const ChainDev* chains, int nchains, int maxN, int team, int nr, int nl, int mode, cudaStream_t st);
 // green_tau: G(tau,tau) into Gnew, G(tau,0), G(0,tau), G(0,0) into gt0, g0t, g00
 // (R = slot nr, L = slot nl); new log weight -> stats[ST_LOGDETM_*]
-void launch_green_tau(const ChainDev* chains, int nchains, int nr, int nl, cudaStream_t st);
+void launch_green_tau(const ChainDev* chains, int nchains, int maxN, int team, int nr, int nl, cudaStream_t st);
 // push_stage (dir 0) / pop_stage (dir 1) of nslots stack slots and G
 void launch_stage(const ChainDev* chains, int nchains, int nslots, int dir, cudaStream_t st);
 void launch_dyn_init(const ChainDev* chains, int nchains, cudaStream_t st);
@@ -72,15 +71,14 @@ void launch_chain_gemm(const ChainDev* chains, int nchains, int maxN, int dst_id
 void launch_dyn_err(const ChainDev* chains, int nchains, cudaStream_t st);
 void launch_zgemm_test(const ChainDev* chains, int nchains, int m, int n, int k, int opa, int opb,
                        int a_id, int b_id, int c_id, double beta_re, cudaStream_t st);
-void launch_qr_test(const ChainDev* chains, int nchains, int a_id, int q_id, cudaStream_t st);
+void launch_qr_test(const ChainDev* chains, int nchains, int maxN, int team, int a_id, int q_id, cudaStream_t st);
 
 // projective path (kern_proj.cu, kern_prop.cu)
-void set_proj_maxN(int maxN);
 // one pass of prog over the N x ne matrix mat_id (right = 1: right multiplications of UL, stored as UL^T)
 void launch_prop_tall(const ChainDev* chains, int nchains, int maxN, int mat_id, const PropProg& prog,
                       int right, int ctas_per_chain, cudaStream_t st);
-void launch_proj_qr(const ChainDev* chains, int nchains, int mat_id, int dst, int add, cudaStream_t st);
-void launch_proj_ulr(const ChainDev* chains, int nchains, int out_id, int logdet, int ia, int ib, cudaStream_t st);
+void launch_proj_qr(const ChainDev* chains, int nchains, int maxN, int team, int mat_id, int dst, int add, cudaStream_t st);
+void launch_proj_ulr(const ChainDev* chains, int nchains, int maxN, int team, int out_id, int logdet, int ia, int ib, cudaStream_t st);
 void launch_proj_green(const ChainDev* chains, int nchains, int inv_id, int dst_id, int ctas, cudaStream_t st);
 void launch_tall_copy(const ChainDev* chains, int nchains, int dst_id, int src_id, cudaStream_t st);
 void launch_proj_update(const ChainDev* chains, int nchains, int nt, int nf, int visit, int dir, int rnd_off,

@@ -7,6 +7,20 @@
 // one chain's matrices (leading dimension N, N <= 512).
 #pragma once
 #include "zgemm.cuh"
+#include "team.cuh"
+
+// C = alpha op(A) op(B) + beta C, the tiles dealt out over the team in the shape
+// that keeps its busiest CTA shortest: a CTA per 64 x 64 tile while there are
+// enough of them, smaller tiles where 64 x 64 leaves CTAs idle (their fragments
+// are re-used less, hence the weights).  Ends with a CTA barrier, not a team one.
+DQ_DEV void team_zgemm(const ZGemmArgs& g, const Team& tm, cplx* smem) {
+    if (tm.size == 1) { zgemm_cta<GemmBig>(g, 0, 1, smem); return; }
+    auto rounds = [&](int bm, int bn) { return (((g.M + bm - 1) / bm) * ((g.N + bn - 1) / bn) + tm.size - 1) / tm.size; };
+    const int c64 = rounds(64, 64) * 64 * 64 * 8, c32 = rounds(64, 32) * 64 * 32 * 9, c16 = rounds(32, 32) * 32 * 32 * 10;
+    if (c64 <= c32 && c64 <= c16) zgemm_cta<GemmBig>(g, tm.rank, tm.size, smem);
+    else if (c32 <= c16) zgemm_cta<Gemm64x32>(g, tm.rank, tm.size, smem);
+    else zgemm_cta<Gemm32x32w>(g, tm.rank, tm.size, smem);
+}
 
 #define QR_NB 16
 // shared memory of a panel: m x 16 with an odd leading dimension (m or m + 1),
@@ -311,28 +325,20 @@ static __device__ void cta_form_q(const double2* A, int N, double2* Qout, Linalg
     }
 }
 
-// X <- Q^H X for all N columns of X (Q from the factored A).
-static __device__ void cta_apply_qh(const double2* A, int N, double2* X, LinalgScratch& sc, cplx* gsm) {
-    for (int p = 0; p < N; p += QR_NB) {
-        const int jb = min(QR_NB, N - p);
-        build_vblock(A, N, p, jb, sc.Vs);
-        const double2* Tp = sc.T + (size_t)(p / QR_NB) * QR_NB * QR_NB;
-        apply_block(sc.Vs, Tp, N, p, jb, X, 0, N, 1, sc, gsm);
-    }
-}
-
-// X <- R^{-1} X with R the upper triangle of A (blocked back substitution).
-static __device__ void trsm_rows16(const double2* A, int N, double2* X, int p0, int p1, cplx* gsm, LinalgSmem* L) {
+// X <- R^{-1} X for rows p0..p1 of X (nc columns, ld N), R the upper triangle of
+// A restricted to them (back substitution in 16-row steps).
+static __device__ void trsm_rows16(const double2* A, int N, double2* X, int nc, int p0, int p1, cplx* gsm, LinalgSmem* L) {
     const int last = p0 + ((p1 - p0 - 1) / QR_NB) * QR_NB;
     for (int p = last; p >= p0; p -= QR_NB) {
         const int jb = min(QR_NB, p1 - p);
         if (p + jb < p1) {
             ZGemmArgs g;
-            g.M = jb; g.N = N; g.K = p1 - p - jb; g.alpha = cmk(-1, 0); g.beta = cmk(1, 0);
+            g.M = jb; g.N = nc; g.K = p1 - p - jb; g.alpha = cmk(-1, 0); g.beta = cmk(1, 0);
             g.A = A + MIDX(p, p + jb, N); g.lda = N; g.opA = OP_N;
             g.B = X + (p + jb); g.ldb = N; g.opB = OP_N;
             g.C = X + p; g.ldc = N;
-            zgemm_cta<GemmWide>(g, 0, 1, gsm);
+            if (nc <= 64) zgemm_cta<Gemm16x64>(g, 0, 1, gsm);
+            else zgemm_cta<GemmWide>(g, 0, 1, gsm);
         }
         // The diagonal is stored as its reciprocal so the solve multiplies.
         for (int e = threadIdx.x; e < jb * jb; e += blockDim.x) {
@@ -341,7 +347,7 @@ static __device__ void trsm_rows16(const double2* A, int N, double2* X, int p0, 
             L->S[a + b * QR_NB] = (a == b) ? cdiv(cmk(1, 0), v) : v;
         }
         __syncthreads();
-        for (int cc = threadIdx.x; cc < N; cc += blockDim.x) {
+        for (int cc = threadIdx.x; cc < nc; cc += blockDim.x) {
             double2 x[QR_NB];
 #pragma unroll
             for (int a = 0; a < QR_NB; ++a) x[a] = (a < jb) ? X[MIDX(p + a, cc, N)] : cmk(0, 0);
@@ -363,10 +369,6 @@ static __device__ void trsm_rows16(const double2* A, int N, double2* X, int p0, 
     }
 }
 
-static __device__ void cta_trsm_upper(const double2* A, int N, double2* X, cplx* gsm, LinalgSmem* L) {
-    trsm_rows16(A, N, X, 0, N, gsm, L);
-}
-
 // ---------------------------------------------------------------------------
 // Two-level blocked QR: 16-wide panels inside 64-wide blocks.  The panels of a
 // block update only the block's own columns; the trailing matrix and the later
@@ -374,57 +376,56 @@ static __device__ void cta_trsm_upper(const double2* A, int N, double2* X, cplx*
 // GEMMs have an inner dimension of 64 instead of 16.  T of a block is built
 // from its panels' triangles: for H = H_a H_b,
 //   T = [[T_a, -T_a (V_a^H V_b) T_b], [0, T_b]].
+// sc.Vs holds the explicit reflectors of the whole factorisation, N x ncol with
+// ld N: a block's unit lower trapezoid with zeros above its diagonal.
+//
+// The work is shared by the CTAs of a team: rank 0 factors each block's panels
+// (a serial chain of small steps that one SM's shared memory holds), and a
+// reflector or a triangle is applied to column chunks that one CTA each owns,
+// because the columns do not depend on one another.  A chunk needs no exchange
+// with the other CTAs from the first reflector to the last, so the team meets
+// twice per 64 columns of the QR and not at all inside Q^H X and R^-1 X.
 // ---------------------------------------------------------------------------
 #define QR_NB2 64
 
-// X <- R^{-1} X, two-level: block rows of 64 are first updated with the solved
-// rows below them by one 64-row GEMM (GemmBig), then solved with the 16-row
-// scheme of trsm_rows16 restricted to the block, so most of the work runs
-// in 64-row DMMA tiles instead of 16-row ones.
-static __device__ void cta_trsm_upper64(const double2* A, int N, double2* X, cplx* gsm, LinalgSmem* L) {
-    const int last64 = ((N - 1) / QR_NB2) * QR_NB2;
-    for (int P = last64; P >= 0; P -= QR_NB2) {
-        const int jb2 = min(QR_NB2, N - P);
-        if (P + jb2 < N) {
-            ZGemmArgs g;
-            g.M = jb2; g.N = N; g.K = N - P - jb2; g.alpha = cmk(-1, 0); g.beta = cmk(1, 0);
-            g.A = A + MIDX(P, P + jb2, N); g.lda = N; g.opA = OP_N;
-            g.B = X + (P + jb2); g.ldb = N; g.opB = OP_N;
-            g.C = X + P; g.ldc = N;
-            zgemm_cta<GemmBig>(g, 0, 1, gsm);
-        }
-        trsm_rows16(A, N, X, P, P + jb2, gsm, L);
-    }
-}
-
-// X[p:N, c0:c0+nc] <- (I - V T V^H)^op X for a jb-wide block (jb <= 64; T ld 64)
-static __device__ void apply_block64(const double2* Vs, const double2* Tp, int N, int p, int jb,
-                                     double2* X, int c0, int nc, int use_th, LinalgScratch& sc, cplx* gsm) {
-    if (nc <= 0) return;
+// X[P:N, c0:c0+nc] <- (I - V T V^H)^op X for a jb-wide block (jb <= 64; T ld 64)
+// whose explicit V (ld N) starts at Vs; the columns' scratch is their own part of
+// sc.Ws and sc.Ws2.
+template <class Cfg>
+static __device__ void apply_block64_cfg(const double2* Vs, const double2* Tp, int N, int p, int jb,
+                                         double2* X, int c0, int nc, int use_th, LinalgScratch& sc, cplx* gsm) {
     const int m = N - p;
+    double2 *w1 = sc.Ws + (size_t)QR_NB2 * c0, *w2 = sc.Ws2 + (size_t)QR_NB2 * c0;
     ZGemmArgs g;
     g.M = jb; g.N = nc; g.K = m; g.alpha = cmk(1, 0); g.beta = cmk(0, 0);
     g.A = Vs; g.lda = N; g.opA = OP_C;
     g.B = X + MIDX(p, c0, N); g.ldb = N; g.opB = OP_N;
-    g.C = sc.Ws; g.ldc = QR_NB2;
-    zgemm_cta<GemmBig>(g, 0, 1, gsm);
+    g.C = w1; g.ldc = QR_NB2;
+    zgemm_cta<Cfg>(g, 0, 1, gsm);
     g.M = jb; g.N = nc; g.K = jb;
     g.A = Tp; g.lda = QR_NB2; g.opA = use_th ? OP_C : OP_N;
-    g.B = sc.Ws; g.ldb = QR_NB2; g.opB = OP_N;
-    g.C = sc.Ws2; g.ldc = QR_NB2;
-    zgemm_cta<GemmBig>(g, 0, 1, gsm);
+    g.B = w1; g.ldb = QR_NB2; g.opB = OP_N;
+    g.C = w2; g.ldc = QR_NB2;
+    zgemm_cta<Cfg>(g, 0, 1, gsm);
     g.M = m; g.N = nc; g.K = jb; g.alpha = cmk(-1, 0); g.beta = cmk(1, 0);
     g.A = Vs; g.lda = N; g.opA = OP_N;
-    g.B = sc.Ws2; g.ldb = QR_NB2; g.opB = OP_N;
+    g.B = w2; g.ldb = QR_NB2; g.opB = OP_N;
     g.C = X + MIDX(p, c0, N); g.ldc = N;
-    zgemm_cta<GemmBig>(g, 0, 1, gsm);
+    zgemm_cta<Cfg>(g, 0, 1, gsm);
+}
+static __device__ void apply_block64(const double2* Vs, const double2* Tp, int N, int p, int jb,
+                                     double2* X, int c0, int nc, int use_th, LinalgScratch& sc, cplx* gsm) {
+    if (nc <= 0) return;
+    if (nc <= 16) apply_block64_cfg<Gemm64x16>(Vs, Tp, N, p, jb, X, c0, nc, use_th, sc, gsm);
+    else if (nc <= 32) apply_block64_cfg<Gemm64x32>(Vs, Tp, N, p, jb, X, c0, nc, use_th, sc, gsm);
+    else apply_block64_cfg<GemmBig>(Vs, Tp, N, p, jb, X, c0, nc, use_th, sc, gsm);
 }
 
 // T (64 x 64, ld 64, zero outside the upper triangle) of the block whose explicit
-// V (jb2 columns, rows from the block's first row, ld N) is in sc.Vs, from the
+// V (jb2 columns, rows from the block's first row, ld N) starts at Vs, from the
 // 16 x 16 triangles of its panels (Tp16, consecutive)
-static __device__ void build_t64(int N, int P, int jb2, const double2* Tp16, double2* T64, LinalgScratch& sc,
-                                 cplx* gsm) {
+static __device__ void build_t64(const double2* Vs, int N, int P, int jb2, const double2* Tp16, double2* T64,
+                                 LinalgScratch& sc, cplx* gsm) {
     const int tid = threadIdx.x, nth = blockDim.x, m = N - P;
     for (int e = tid; e < QR_NB2 * QR_NB2; e += nth) {
         const int a = e % QR_NB2, b = e / QR_NB2;
@@ -436,10 +437,10 @@ static __device__ void build_t64(int N, int P, int jb2, const double2* Tp16, dou
         const double2* Tb = Tp16 + (size_t)(k / QR_NB) * QR_NB * QR_NB;
         ZGemmArgs g;   // X = V_a^H V_b  (k x jb)
         g.M = k; g.N = jb; g.K = m; g.alpha = cmk(1, 0); g.beta = cmk(0, 0);
-        g.A = sc.Vs; g.lda = N; g.opA = OP_C;
-        g.B = sc.Vs + (size_t)k * N; g.ldb = N; g.opB = OP_N;
+        g.A = Vs; g.lda = N; g.opA = OP_C;
+        g.B = Vs + (size_t)k * N; g.ldb = N; g.opB = OP_N;
         g.C = sc.Ws; g.ldc = QR_NB2;
-        zgemm_cta<GemmBig>(g, 0, 1, gsm);
+        zgemm_cta<Gemm64x16>(g, 0, 1, gsm);
         // Y = T_a X (T_a upper triangular), then T(0:k, k:k+jb) = -Y T_b, with
         // T_a (k x k, ld k), X and Y (k x jb, ld k) and T_b staged in shared
         // memory (the GEMM staging buffer: k^2 + 2 k QR_NB + QR_NB^2 <= 4096
@@ -474,60 +475,108 @@ static __device__ void build_t64(int N, int P, int jb2, const double2* Tp16, dou
 }
 
 // In-place QR of the first ncol columns of A (ld N), two-level blocked; R above
-// the diagonal, reflectors below, tau, panel triangles in sc.T and block
-// triangles in sc.T64.  smem_panel holds >= QR_PANEL_ELEMS(N) double2.
+// the diagonal, reflectors below and, explicit, in sc.Vs, tau, panel triangles in
+// sc.T and block triangles in sc.T64.  smem_panel holds >= QR_PANEL_ELEMS(N)
+// double2.  Every CTA of the team calls it; the results are visible to all on return.
 static __device__ void cta_qr64(double2* A, int N, LinalgScratch& sc, double2* smem_panel, cplx* gsm, LinalgSmem* L,
-                                int ncol = -1) {
+                                const Team& tm, int ncol = -1) {
     if (ncol < 0) ncol = N;
     for (int P = 0; P < ncol; P += QR_NB2) {
         const int jb2 = min(QR_NB2, ncol - P);
-        for (int p = P; p < P + jb2; p += QR_NB) {
-            const int jb = min(QR_NB, P + jb2 - p), m = N - p, ldp = m + ((m & 1) ^ 1);
-            double2* Pn = smem_panel;
-            for (int e = threadIdx.x; e < m * jb; e += blockDim.x) {
-                int r = e % m, cc = e / m;
-                Pn[(size_t)cc * ldp + r] = A[MIDX(p + r, p + cc, N)];
-            }
-            __syncthreads();
-            panel_qr(Pn, m, ldp, jb, sc.tau + p, L);
-            double2* Tp = sc.T + (size_t)(p / QR_NB) * QR_NB * QR_NB;
-            panel_larft(Pn, m, ldp, jb, sc.tau + p, Tp, L);
-            for (int e = threadIdx.x; e < m * jb; e += blockDim.x) {
-                int r = e % m, cc = e / m;
-                A[MIDX(p + r, p + cc, N)] = Pn[(size_t)cc * ldp + r];
-                sc.Vs[MIDX(r, cc, N)] = (r < cc) ? cmk(0, 0) : (r == cc) ? cmk(1, 0) : Pn[(size_t)cc * ldp + r];
-            }
-            __syncthreads();
-            if (p + jb < P + jb2) apply_block(sc.Vs, Tp, N, p, jb, A, p + jb, P + jb2 - p - jb, 1, sc, gsm);
-        }
-        build_vblock(A, N, P, jb2, sc.Vs);
+        double2* VP = sc.Vs + MIDX(P, P, N);
         double2* T64 = sc.T64 + (size_t)(P / QR_NB2) * QR_NB2 * QR_NB2;
-        build_t64(N, P, jb2, sc.T + (size_t)(P / QR_NB) * QR_NB * QR_NB, T64, sc, gsm);
-        if (P + jb2 < ncol) apply_block64(sc.Vs, T64, N, P, jb2, A, P + jb2, ncol - P - jb2, 1, sc, gsm);
+        if (tm.rank == 0) {
+            for (int p = P; p < P + jb2; p += QR_NB) {
+                const int jb = min(QR_NB, P + jb2 - p), m = N - p, ldp = m + ((m & 1) ^ 1);
+                double2* Pn = smem_panel;
+                for (int e = threadIdx.x; e < m * jb; e += blockDim.x) {
+                    int r = e % m, cc = e / m;
+                    Pn[(size_t)cc * ldp + r] = A[MIDX(p + r, p + cc, N)];
+                }
+                __syncthreads();
+                panel_qr(Pn, m, ldp, jb, sc.tau + p, L);
+                double2* Tp = sc.T + (size_t)(p / QR_NB) * QR_NB * QR_NB;
+                panel_larft(Pn, m, ldp, jb, sc.tau + p, Tp, L);
+                for (int e = threadIdx.x; e < m * jb; e += blockDim.x) {
+                    int r = e % m, cc = e / m;
+                    A[MIDX(p + r, p + cc, N)] = Pn[(size_t)cc * ldp + r];
+                    sc.Vs[MIDX(p + r, p + cc, N)] = (r < cc) ? cmk(0, 0) : (r == cc) ? cmk(1, 0) : Pn[(size_t)cc * ldp + r];
+                }
+                for (int e = threadIdx.x; e < (p - P) * jb; e += blockDim.x)     // above the panel, inside the block
+                    sc.Vs[MIDX(P + e % (p - P), p + e / (p - P), N)] = cmk(0, 0);
+                __syncthreads();
+                if (p + jb < P + jb2)
+                    apply_block(sc.Vs + MIDX(p, p, N), Tp, N, p, jb, A, p + jb, P + jb2 - p - jb, 1, sc, gsm);
+            }
+            build_t64(VP, N, P, jb2, sc.T + (size_t)(P / QR_NB) * QR_NB * QR_NB, T64, sc, gsm);
+        }
+        tm.sync();
+        const int nc = ncol - P - jb2, w = tm.chunk(nc);
+        if (nc > 0) {
+            for (int c = tm.rank * w; c < nc; c += tm.size * w)
+                apply_block64(VP, T64, N, P, jb2, A, P + jb2 + c, min(w, nc - c), 1, sc, gsm);
+            tm.sync();
+        }
     }
 }
 
-// The first ncol columns of Q (ld N) from cta_qr64's factors into Qout.
-static __device__ void cta_form_q64(const double2* A, int N, double2* Qout, LinalgScratch& sc, cplx* gsm, int ncol = -1) {
+// The first ncol columns of Q (ld N) from cta_qr64's factors into Qout; each
+// CTA of the team forms its own column chunks (no team barrier).
+static __device__ void cta_form_q64(int N, double2* Qout, LinalgScratch& sc, cplx* gsm, const Team& tm, int ncol = -1) {
     if (ncol < 0) ncol = N;
-    for (int e = threadIdx.x; e < N * ncol; e += blockDim.x) {
-        int r = e % N, cc = e / N;
-        Qout[e] = cmk(r == cc ? 1.0 : 0.0, 0.0);
-    }
-    __syncthreads();
-    const int last = ((ncol - 1) / QR_NB2) * QR_NB2;
-    for (int P = last; P >= 0; P -= QR_NB2) {
-        const int jb2 = min(QR_NB2, ncol - P);
-        build_vblock(A, N, P, jb2, sc.Vs);
-        apply_block64(sc.Vs, sc.T64 + (size_t)(P / QR_NB2) * QR_NB2 * QR_NB2, N, P, jb2, Qout, P, ncol - P, 0, sc, gsm);
+    const int w = tm.chunk(ncol);
+    for (int c = tm.rank * w; c < ncol; c += tm.size * w) {
+        const int nc = min(w, ncol - c);
+        double2* X = Qout + MIDX(0, c, N);
+        for (int e = threadIdx.x; e < N * nc; e += blockDim.x)
+            X[e] = cmk((e % N) == c + e / N ? 1.0 : 0.0, 0.0);
+        __syncthreads();
+        // block P leaves the unit columns before it as they are
+        for (int P = ((c + nc - 1) / QR_NB2) * QR_NB2; P >= 0; P -= QR_NB2) {
+            const int jb2 = min(QR_NB2, ncol - P), lo = max(c, P);
+            apply_block64(sc.Vs + MIDX(P, P, N), sc.T64 + (size_t)(P / QR_NB2) * QR_NB2 * QR_NB2, N, P, jb2, Qout, lo,
+                          c + nc - lo, 0, sc, gsm);
+        }
     }
 }
 
-// X <- Q^H X for all N columns of X (Q from cta_qr64 of an N x N matrix).
-static __device__ void cta_apply_qh64(const double2* A, int N, double2* X, LinalgScratch& sc, cplx* gsm) {
-    for (int P = 0; P < N; P += QR_NB2) {
+// Columns c0 .. c0+nc of X <- Q^H X (Q from cta_qr64 of an N x N matrix); one CTA.
+static __device__ void cta_apply_qh64(int N, double2* X, int c0, int nc, LinalgScratch& sc, cplx* gsm) {
+    for (int P = 0; P < N; P += QR_NB2)
+        apply_block64(sc.Vs + MIDX(P, P, N), sc.T64 + (size_t)(P / QR_NB2) * QR_NB2 * QR_NB2, N, P, min(QR_NB2, N - P),
+                      X, c0, nc, 1, sc, gsm);
+}
+
+// Columns c0 .. c0+nc of X <- R^{-1} X, two-level; one CTA: block rows of 64 are
+// first updated with the solved rows below them by one 64-row GEMM, then solved
+// with the 16-row scheme of trsm_rows16 restricted to the block, so most of the
+// work runs in 64-row DMMA tiles instead of 16-row ones.
+static __device__ void cta_trsm_upper64(const double2* A, int N, double2* X, int c0, int nc, cplx* gsm, LinalgSmem* L) {
+    const int last64 = ((N - 1) / QR_NB2) * QR_NB2;
+    X += MIDX(0, c0, N);
+    for (int P = last64; P >= 0; P -= QR_NB2) {
         const int jb2 = min(QR_NB2, N - P);
-        build_vblock(A, N, P, jb2, sc.Vs);
-        apply_block64(sc.Vs, sc.T64 + (size_t)(P / QR_NB2) * QR_NB2 * QR_NB2, N, P, jb2, X, 0, N, 1, sc, gsm);
+        if (P + jb2 < N) {
+            ZGemmArgs g;
+            g.M = jb2; g.N = nc; g.K = N - P - jb2; g.alpha = cmk(-1, 0); g.beta = cmk(1, 0);
+            g.A = A + MIDX(P, P + jb2, N); g.lda = N; g.opA = OP_N;
+            g.B = X + (P + jb2); g.ldb = N; g.opB = OP_N;
+            g.C = X + P; g.ldc = N;
+            if (nc <= 16) zgemm_cta<Gemm64x16>(g, 0, 1, gsm);
+            else if (nc <= 32) zgemm_cta<Gemm64x32>(g, 0, 1, gsm);
+            else zgemm_cta<GemmBig>(g, 0, 1, gsm);
+        }
+        trsm_rows16(A, N, X, nc, P, P + jb2, gsm, L);
+    }
+}
+
+// X <- R^{-1} Q^H X on the team's column chunks (no team barrier)
+static __device__ void cta_solve64(const double2* A, int N, double2* X, LinalgScratch& sc, cplx* gsm, LinalgSmem* L,
+                                   const Team& tm) {
+    const int w = tm.chunk(N);
+    for (int c = tm.rank * w; c < N; c += tm.size * w) {
+        const int nc = min(w, N - c);
+        cta_apply_qh64(N, X, c, nc, sc, gsm);
+        cta_trsm_upper64(A, N, X, c, nc, gsm, L);
     }
 }

@@ -217,6 +217,11 @@ __device__ void zgemm_cta(const ZGemmArgs& g, int tile0, int tstep, cplx* smem) 
 typedef ZGemmCfg<64, 64, 16, 2, 4> GemmBig;     // square-ish products
 typedef ZGemmCfg<32, 64, 16, 2, 4> GemmMid;     // panels with M <= 32
 typedef ZGemmCfg<16, 128, 16, 1, 8> GemmWide;   // M = 16 rows (reflector blocks)
+typedef ZGemmCfg<16, 64, 16, 1, 8> Gemm16x64;   // M = 16 rows, up to 64 columns
+// narrow column chunks and single tiles of a matrix that a team of CTAs shares
+typedef ZGemmCfg<64, 32, 16, 4, 2> Gemm64x32;
+typedef ZGemmCfg<64, 16, 16, 8, 1> Gemm64x16;
+typedef ZGemmCfg<32, 32, 16, 4, 2> Gemm32x32w;  // 8 warps on 32 x 32
 // small shapes whose sides are multiples of 16 or 48 (the projective update's
 // window GEMMs: window rows 32, ne = 144 at the benchmark size)
 typedef ZGemmCfg<48, 48, 16, 3, 2> Gemm48x48;

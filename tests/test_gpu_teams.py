@@ -1,0 +1,63 @@
+"""Teams of CTAs (thread-block clusters) on one chain: the number of chains of a
+handle sets the team size (16 CTAs per chain for a few chains, one per chain for
+hundreds), and the chains' sizes set how columns and tiles are dealt out over a
+team.  Handles of mixed sizes at every team size: the QR against its defining
+properties (the bounds of test_qr_householder), start-up and one sweep against
+the oracle (fields and accept counts exactly, G to 1e-10)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+# one column chunk of a team and its remainders: below 16, past 16, 64 and 128 columns
+LENGTHS = (8, 34, 66, 98, 130)
+CHAINS = (1, 6, 14, 40, 160)
+
+
+def params(l):
+    return dict(lattice=3, l1=l, l2=1, beta=1.2, dtau=0.1, rhub=3.0, nflr=2, kinetic=0, update=1, hs=1, nwrap=5,
+                nublock=16)
+
+
+def handle(sb, n):
+    ps = [sb.DqmcParams.make(**params(l)) for l in (LENGTHS if n > 1 else LENGTHS[-1:])]
+    return sb.Dqmc([ps[c % len(ps)] for c in range(n)], n_chains=n, seeds=[sb.test_seed(c) for c in range(n)])
+
+
+@pytest.mark.parametrize("n", CHAINS)
+def test_qr(sb, n):
+    with handle(sb, n) as g:
+        rng = np.random.default_rng(n)
+        As = []
+        for c in range(min(n, 5)):
+            N = g.ndim(c)
+            A = (rng.standard_normal((N, N)) + 1j * rng.standard_normal((N, N))) * np.logspace(8, -8, N)[None, :]
+            g.set_work(0, A, c)
+            As.append(A)
+        ld = g.test_qr(0, 1)
+        for c, A in enumerate(As):
+            Q, R = g.work(1, c), np.triu(g.work(0, c))
+            assert np.max(np.abs(Q.conj().T @ Q - np.eye(len(A)))) < 1e-12
+            assert np.max(np.abs(Q @ R - A) / np.max(np.abs(A), axis=0)[None, :]) < 1e-12
+            sign, _ = np.linalg.slogdet(Q)
+            assert abs(np.exp(1j * ld[c].imag) - sign) < 1e-10 and abs(ld[c].real) < 1e-10
+
+
+@pytest.mark.parametrize("n", CHAINS)
+def test_sweep(sb, oracle, n):
+    with handle(sb, n) as g:
+        g.sweep_start()
+        chains = range(min(n, 5))
+        ch = []
+        for c in chains:
+            m = oracle.Model(**params(g.ndim(c)))
+            o = oracle.Chain(m, sb.test_seed(c))
+            o.sweep_start()
+            assert np.max(np.abs(g.green(c) - o.green())) < 1e-10
+            ch.append((m, o))
+        g.sweep_b0(); g.sweep_0b()
+        for c, (m, o) in zip(chains, ch):
+            o.sweep_b0(); o.sweep_0b()
+            assert np.array_equal(g.conf(c), o.conf())
+            assert g.diag(c)["accepted"] == o.diag()["accepted"]
+            assert np.max(np.abs(g.green(c) - o.green())) < 1e-10
