@@ -1147,7 +1147,9 @@ struct dqmc_handle {
     std::vector<void*> allocs;
     cudaStream_t st = nullptr;
     int nch = 0, maxN = 0, ltrot = 0, nst = 0, nwrap = 0, nnf_max = 0;
+    int max_nublock = 1;             // largest flush depth of the models
     int team = 1;                    // CTAs per chain of the QR and Green's function kernels
+    int uteam = 1;                   // and of the update kernel
     int started = 0;
     cudaGraphExec_t sweep_graph = nullptr;
     int graph_meas = -1;
@@ -1288,6 +1290,7 @@ extern "C" int dqmc_gpu_create(const dqmc_params* params, int n_params, int n_ch
         h->nnf_max = std::max(h->nnf_max, m->nn_nf);
         h->maxNe = std::max(h->maxNe, m->p.ne);
         h->max_lq = std::max(h->max_lq, m->lq);
+        h->max_nublock = std::max(h->max_nublock, m->nublock_dev);
     }
     {
         const dqmc_params& p0 = h->models[0]->p;
@@ -1452,6 +1455,10 @@ extern "C" int dqmc_gpu_create(const dqmc_params* params, int n_params, int n_ch
         cudaMemcpy(h->d_chains, v.data(), sizeof(ChainDev) * n_chains, cudaMemcpyHostToDevice);
     }
     h->team = pick_team(n_chains);
+    // the update of up to about two windows of sites is its serial walk: 50.6 us a
+    // slice with 4 to 16 CTAs and 52.0 us with one for a chain of 64 sites, 26.9 us
+    // with one and 28.7 us with 8 for 16 sites; at 100 sites 132 us against 192 us
+    h->uteam = h->maxN > 64 ? h->team : 1;
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
     h->ctas_per_chain = std::max(1, std::min(h->maxN / 16, (2 * sms + n_chains - 1) / n_chains));
@@ -2091,7 +2098,7 @@ static void enqueue_b0(dqmc_handle* h, int lupdate, int lmeasure) {
         tmark(h, DQMC_PROF_PROP_L);
         launch_prog(h, MAT_G, pr, 1);
         tmark(h, DQMC_PROF_PROP_R);
-        if (lupdate && m.p.rhub != 0.0) { launch_update(h->d_chains, h->nch, nt, visit, h->st, 0, 1); tmark(h, DQMC_PROF_UPDATE); }
+        if (lupdate && m.p.rhub != 0.0) { launch_update(h->d_chains, h->nch, h->max_nublock, h->uteam, nt, visit, h->st, 0, 1); tmark(h, DQMC_PROF_UPDATE); }
         pl.n = 0; pr.n = 0;
         prog_v(m, pl, PW_INV, nt);         // u left_backward
         prog_v(m, pr, PW_FWD, nt);         // u right_forward
@@ -2181,7 +2188,7 @@ static void enqueue_0b(dqmc_handle* h, int lupdate, int lmeasure) {
         tmark(h, DQMC_PROF_PROP_L);
         launch_prog(h, MAT_G, pr, 1);
         tmark(h, DQMC_PROF_PROP_R);
-        if (lupdate && m.p.rhub != 0.0) { launch_update(h->d_chains, h->nch, nt, visit, h->st); tmark(h, DQMC_PROF_UPDATE); }
+        if (lupdate && m.p.rhub != 0.0) { launch_update(h->d_chains, h->nch, h->max_nublock, h->uteam, nt, visit, h->st); tmark(h, DQMC_PROF_UPDATE); }
         pl.n = 0; pr.n = 0;
         prog_k(m, pl, PW_FWD, 1);
         prog_k(m, pr, PW_INV, 1);
@@ -2760,10 +2767,10 @@ extern "C" int dqmc_gpu_update(dqmc_handle* h, int nt) {
         // exactly the 2 N draws of uconf%update (the slice layout of a sweep also
         // holds the plaquette and bond words); the U words start the b0 layout
         launch_sfmt(h->d_chains, h->nch, -2 * m0.N, h->st);
-        launch_update(h->d_chains, h->nch, nt, 0, h->st, 0, 1);
+        launch_update(h->d_chains, h->nch, h->max_nublock, h->uteam, nt, 0, h->st, 0, 1);
     } else {
         launch_sfmt(h->d_chains, h->nch, 1, h->st);
-        launch_update(h->d_chains, h->nch, nt, 0, h->st);
+        launch_update(h->d_chains, h->nch, h->max_nublock, h->uteam, nt, 0, h->st);
     }
     CK(cudaStreamSynchronize(h->st));
     CK(cudaGetLastError());
@@ -2793,7 +2800,7 @@ extern "C" int dqmc_gpu_time_op(dqmc_handle* h, int op, int reps, double* ms_out
     int spare = h->nst + 1;
     auto enqueue = [&]() {
         switch (op) {
-        case 0: launch_update(h->d_chains, h->nch, 1, 0, h->st); break;
+        case 0: launch_update(h->d_chains, h->nch, h->max_nublock, h->uteam, 1, 0, h->st); break;
         case 1: launch_stab_slots(h->d_chains, h->nch, h->maxN, h->team, 0, spare, h->st); break;
         case 2: launch_green(h->d_chains, h->nch, h->maxN, h->team, 1, 0, 0, h->st); break;
         case 3: { PropProg p; p.n = 0; prog_k(m, p, PW_INV, 0); prog_v(m, p, PW_INV, 1); prog_k(m, p, PW_INV, 1);
@@ -3371,7 +3378,7 @@ static void block_move(dqmc_handle* h, dqmc_nn* nn, int t0) {
     launch_nn_forward(nn_w(nn), in, 2 * nch, h->d_S, nullptr, nullptr, h->st);
     launch_blk_begin(h->d_chains, nch, h->d_S, h->d_u, t0, NN_BLK_T, h->st);
     for (int j = 0; j < NN_BLK_T; ++j) {
-        launch_update(h->d_chains, nch, t0 + j, 0, h->st, 1);
+        launch_update(h->d_chains, nch, h->max_nublock, h->uteam, t0 + j, 0, h->st, 1);
         if (j + 1 < NN_BLK_T) {
             PropProg pl; pl.n = 0; PropProg pr; pr.n = 0;
             prog_k(m, pl, PW_FWD, 1); prog_k(m, pl, PW_FWD, 0); prog_v(m, pl, PW_FWD, t0 + j + 1);
@@ -3419,7 +3426,7 @@ static void enqueue_0b_blocks(dqmc_handle* h, dqmc_nn* nn, int lupdate, int lmea
         launch_prog(h, MAT_G, pl, 0);
         launch_prog(h, MAT_G, pr, 1);
         if (start[nt]) block_move(h, nn, nt);
-        if (lupdate) launch_update(h->d_chains, h->nch, nt, visit, h->st);
+        if (lupdate) launch_update(h->d_chains, h->nch, h->max_nublock, h->uteam, nt, visit, h->st);
         pl.n = 0; pr.n = 0;
         prog_k(m, pl, PW_FWD, 1);
         prog_k(m, pr, PW_INV, 1);

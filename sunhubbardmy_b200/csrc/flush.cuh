@@ -6,10 +6,10 @@
 typedef GemmBig UpdGemm;
 
 // G += A B^T over the first K columns of the N x nb factors (alpha = beta = 1),
-// every output tile by this CTA: the accumulators start from the G tile (read
+// the output tiles tile0, tile0 + tstep, ... by this CTA: the accumulators start from the G tile (read
 // while the first A and B stages are in flight) and are stored straight back,
 // so the epilogue needs no shared-memory pass and no second read of G.
-DQ_DEV void flush_addto(double2* G, const double2* A, const double2* B, int N, int K, cplx* smem) {
+DQ_DEV void flush_addto(double2* G, const double2* A, const double2* B, int N, int K, cplx* smem, int tile0, int tstep) {
     typedef UpdGemm Cfg;
     constexpr int BM = Cfg::BM, BN = Cfg::BN, BK = Cfg::BK, FM = Cfg::FM, FN = Cfg::FN;
     const int tid = threadIdx.x, nthr = blockDim.x;
@@ -25,7 +25,7 @@ DQ_DEV void flush_addto(double2* G, const double2* A, const double2* B, int N, i
     cplx* As1 = smem + Cfg::SA + Cfg::SB;
     cplx* Bs1 = smem + 2 * Cfg::SA + Cfg::SB;
     const int nk = (K + BK - 1) / BK;
-    for (int t = 0; t < ntiles; ++t) {
+    for (int t = tile0; t < ntiles; t += tstep) {
         const int m0 = (t % tm) * BM, n0 = (t / tm) * BN;
         zgemm_load_stage<Cfg>(g, m0, n0, 0, As0, Bs0, tid, nthr);
         cp_async_commit();

@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(PLQ_NT, 2) k_plq_delay(const ChainDev* __restr
             if (k) plq_rows(A, N, k, pc, z, Mi);
         }
         if (k > 0 && (k + z > nbv || kp == lq - 1)) {
-            flush_addto(G, A, B, N, k, dsm);
+            flush_addto(G, A, B, N, k, dsm, 0, 1);
             k = 0;
         }
     }
