@@ -2077,7 +2077,7 @@ static void launch_plq(dqmc_handle* h, int nt, int visit, int dir, int lupdate) 
 static void launch_vbond(dqmc_handle* h, int nt, int nf, int visit, int dir) {
     int nbmin = 64;
     for (const HostModel* m : h->models) nbmin = std::min(nbmin, m->nublock_dev);
-    if (!launch_vbond_delay(h->d_chains, h->nch, nbmin, nt, nf, visit, dir, h->st))
+    if (!launch_vbond_delay(h->d_chains, h->nch, nbmin, h->uteam, nt, nf, visit, dir, h->st))
         launch_vbond_slice(h->d_chains, h->nch, h->maxN, nt, nf, visit, dir, h->st);
 }
 

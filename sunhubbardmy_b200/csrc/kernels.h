@@ -26,7 +26,7 @@ void launch_vbond_slice(const ChainDev* chains, int nchains, int maxN, int nt, i
                         cudaStream_t st);
 // the same, delayed (rank-2 columns flushed by a DMMA GEMM); returns 0 without
 // launching when nublock leaves fewer than two delayed columns
-int launch_vbond_delay(const ChainDev* chains, int nchains, int nublock, int nt, int nf, int visit, int dir,
+int launch_vbond_delay(const ChainDev* chains, int nchains, int nublock, int team, int nt, int nf, int visit, int dir,
                        cudaStream_t st);
 // the same delayed (lupdate = 1; the accepted changes flushed by a DMMA GEMM);
 // returns 0 without launching when nublock < z

@@ -35,6 +35,14 @@ DQ_DEV void dmma(double& d0, double& d1, double a, double b) {
         : "+d"(d0), "+d"(d1) : "d"(a), "d"(b));
 }
 
+// c += a b on one 8 x 8 tile of complex accumulators (one k step of 4)
+DQ_DEV void zdmma(double (&cr)[2], double (&ci)[2], cplx a, cplx b) {
+    dmma(cr[0], cr[1], a.x, b.x);
+    dmma(ci[0], ci[1], a.x, b.y);
+    dmma(cr[0], cr[1], -a.y, b.y);
+    dmma(ci[0], ci[1], a.y, b.x);
+}
+
 DQ_DEV void cp_async16(void* smem, const void* gmem, bool valid) {
     unsigned s = (unsigned)__cvta_generic_to_shared(smem);
     int n = valid ? 16 : 0;
