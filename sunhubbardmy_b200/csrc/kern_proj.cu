@@ -13,11 +13,11 @@
 //    windows of `wrows` rows (nustock): the window's rows of R = UR ULRINV and
 //    of F = R UL are formed by two GEMMs, the accept/reject sequence runs on
 //    the F block in shared memory while Gamma^-1 = (I + Delta F_AA)^-1 Delta
-//    is bordered one accepted unit at a time, and the window is flushed with
+//    is built up one accepted unit at a time, and the window is flushed with
 //    ULRINV -= (ULRINV UL_A)(Gamma^-1 R_A) and UR_A <- (I + Delta) UR_A.
 //    Instead of re-evaluating F_rr - F_rA Gamma^-1 F_Ar for each unit, the
-//    kernel keeps the trailing block of F updated (rank-2 Schur complement
-//    per accept), which gives the same numbers in exact arithmetic.
+//    walk keeps the Schur complement of F as a sum of products (pwin_walk),
+//    which gives the same numbers in exact arithmetic.
 //  * k_proj_qr: s_zgeQR_pqmc (lib/s_matrix.f90:1822-1996) as used by
 //    dqmc_proj_stablize_0b_qr / _b0_qr: Q of a tall N x ne matrix with an
 //    even number of negative R diagonal entries (else column 1 is negated)
@@ -34,6 +34,7 @@
 
 #define PW_MAXR 32          // largest update window (rows)
 #define PW_LD (PW_MAXR + 1)
+#define PW_LS (PW_MAXR + 2)   // pitch of what the DMMA fragments read: 2 (mod 8)
 
 struct ProjSmem {
     LinalgSmem L;
@@ -205,21 +206,13 @@ __global__ void k_tall_copy(const ChainDev* __restrict__ chains, int dst_id, int
 // walker.  Scratch per walker in pw: Rg (nr x ne), Fg, Gg (nr x nr), Ut, Vt.
 // ---------------------------------------------------------------------------
 struct PUpdSmem {
-    double2 F[PW_MAXR * PW_LD];     // F block of the window (window-start values)
-    double2 Pc[PW_MAXR * PW_LD];    // F block with the window's accepted changes folded in
-    double2 Gm[PW_MAXR * PW_LD];    // Gamma^-1 in window coordinates (zero off the accepted rows)
-    double2 colr[PW_MAXR * 2], rowr[PW_MAXR * 2], ikk[PW_MAXR * 2], kik[PW_MAXR * 2];
-    double2 gkk[4];
-    double2 dl[PW_MAXR];
-    double2 phase;
+    double2 F[PW_MAXR * PW_LD];     // F(x, y) of the window at x + y * PW_LD (window-start values)
+    // vectors of the accepted rows m, element of window row x at m * PW_LS + x (see pwin_walk)
+    double2 aP[PW_MAXR * PW_LS], bP[PW_MAXR * PW_LS], al[PW_MAXR * PW_LS], be[PW_MAXR * PW_LS];
+    double2 Gm[PW_MAXR * PW_LS];    // Gamma(x, y) at x + y * PW_LS (zero off the accepted rows)
+    double2 dl[PW_MAXR];            // Delta of the accepted rows, else 0
     int rows[PW_MAXR];
-    int accr[PW_MAXR];
-    int acc_flag[2], nacc;
-    double accm, nties;
-    // per-unit proposal, prepared in parallel before the sequential walk
-    double2 ud1[PW_MAXR], ud2[PW_MAXR];   // Delta of the unit's rows
-    double ur2[PW_MAXR];                  // accept threshold (second draw)
-    int uisp[PW_MAXR], ukk[PW_MAXR];      // proposed value, HS-table index (site field)
+    int nacc;                       // accepted rows
 };
 
 DQ_DEV double u32_stream(uint32_t u) { return ((double)u + 0.5) * (1.0 / 4294967296.0); }
@@ -299,10 +292,155 @@ __global__ void __launch_bounds__(256) k_pwin_flush(const ChainDev* __restrict__
     for (int t = blockIdx.x; t < nt; t += gridDim.x) zgemm_tile(g, cl, t, ssm);
 }
 
+// The accept / reject walk of a window, by one warp: lane x holds row x of the
+// window and the b x b diagonal block of its unit in
+//   P = F - F Gamma F = F - sum_m a_m b_m,
+// so every remaining unit is tested at once and the first that passes (a ballot)
+// is accepted, as the sequential visit does.  An accepted unit with rows r and
+// g = (I + Delta P_rr)^-1 Delta appends, per row,
+//   a = P(:, r) g, b = P(r, :),  al = (e_r - Gamma F(:, r)) g, be = e_r - F(r, :) Gamma,
+// all four by the same recursion over the m accepted rows (coefficients b_m(r) and
+// a_m(r)), and Gamma = sum_m al_m be_m.  No block barrier inside the walk: with two of
+// them a unit and one thread's divisions it took about 100 of the 171 us that a window of
+// 64 walkers (32 rows, ne = 144) lasted.
+template <int B>
+DQ_DEV void pwin_walk(PUpdSmem* S, const ChainDev& c, const ModelDev& md, const uint32_t* rnd, int32_t* cf, int u0, int nu) {
+    const int lane = threadIdx.x & 31, k = lane / B, x = lane, lc = B == 2 ? 2 : md.lcomp;
+    const bool live = k < nu, lead = live && lane % B == 0;
+    double2 ph = cmk(c.stats[ST_PHASE_RE], c.stats[ST_PHASE_IM]);
+    double2 d1 = cmk(0, 0), d2 = cmk(0, 0), phr = cmk(1, 0), p0 = cmk(0, 0), p1 = cmk(0, 0);
+    double thr = 0.0, gam = 1.0;
+    int isp = 0;
+    bool cand = live;
+    if (live) {
+        const int u = u0 + k, is = cf[u];
+        const int iflip = (int)ceil(u32_stream(rnd[2 * u]) * (lc - 1));
+        isp = (is + iflip - 1) % lc + 1;
+        thr = u32_stream(rnd[2 * u + 1]);
+        if (B == 2) {
+            d1 = md.vdp[is - 1];
+            d2 = md.vdm[is - 1];
+            p1 = S->F[x + (x ^ 1) * PW_LD];
+        } else {
+            const int kk = (is - 1) * (lc - 1) + (iflip - 1);
+            d1 = md.delta[kk];
+            gam = md.gam_ratio[kk];
+            phr = md.phase_ratio[kk];
+        }
+        p0 = S->F[x + x * PW_LD];
+    }
+    S->dl[lane] = cmk(0, 0);
+    double accm = 0.0;
+    int pc = 0, nm = 0, nties = 0;
+    while (pc < nu) {
+        // the unit's ratio and g, in every lane of the unit
+        double2 det, g11, g12 = cmk(0, 0), g21 = cmk(0, 0), g22 = cmk(0, 0);
+        if (B == 2) {
+            const double2 o0 = cmk(__shfl_xor_sync(0xffffffffu, p0.x, 1), __shfl_xor_sync(0xffffffffu, p0.y, 1));
+            const double2 o1 = cmk(__shfl_xor_sync(0xffffffffu, p1.x, 1), __shfl_xor_sync(0xffffffffu, p1.y, 1));
+            const bool first = (lane & 1) == 0;
+            const double2 prr = first ? p0 : o0, pr1 = first ? p1 : o1, p1r = first ? o1 : p1, p11 = first ? o0 : p0;
+            const double2 v11 = cadd(cmk(1, 0), cmul(prr, d1)), v21 = cmul(p1r, d1);
+            const double2 v12 = cmul(pr1, d2), v22 = cadd(cmk(1, 0), cmul(p11, d2));
+            det = csub(cmul(v11, v22), cmul(v12, v21));
+            const double2 id = cdiv(cmk(1, 0), det);
+            g11 = cmul(cmul(v22, d1), id);
+            g12 = cmul(cmul(cmk(-v12.x, -v12.y), d1), id);
+            g21 = cmul(cmul(cmk(-v21.x, -v21.y), d2), id);
+            g22 = cmul(cmul(v11, d2), id);
+        } else {
+            const double2 ratio1 = cadd(cmk(1, 0), cmul(p0, d1));
+            double2 r = ratio1;
+            for (int f = 1; f < md.nflr; ++f) r = cmul(r, ratio1);
+            det = cmul(cscale(r, gam), phr);
+            g11 = cdiv(d1, ratio1);
+        }
+        const double num = fabs(cmul(det, ph).x), ax = fabs(ph.x), lim = thr * ax;
+        const bool open = cand && k >= pc;
+        const bool pass = open && num > lim;
+        const unsigned bal = __ballot_sync(0xffffffffu, pass);
+        const int kf = bal ? (__ffs(bal) - 1) / B : nu;
+        nties += lead && open && k <= kf && fabs(num - lim) < DQ_NEAR_TIE * ax;
+        if (!bal) break;
+        const int r = kf * B;
+        auto from = [&](double2 v) { return cmk(__shfl_sync(0xffffffffu, v.x, r), __shfl_sync(0xffffffffu, v.y, r)); };
+        det = from(det);
+        g11 = from(g11);
+        if (B == 2) { g12 = from(g12); g21 = from(g21); g22 = from(g22); }
+        ph = cmul(ph, det);
+        ph = cscale(ph, 1.0 / sqrt(cabs2(ph)));
+        accm += 1.0;
+        if (k == kf) {
+            cand = false;
+            S->dl[lane] = lane % B == 0 ? d1 : d2;
+            if (lane % B == 0) cf[u0 + k] = isp;
+        }
+        // P(x, r + q), P(r + q, x), (e - Gamma F)(x, r + q), (e - F Gamma)(r + q, x)
+        double2 cc[B], rr[B], aa[B], bb[B];
+#pragma unroll
+        for (int q = 0; q < B; ++q) {
+            cc[q] = S->F[x + (r + q) * PW_LD];
+            rr[q] = S->F[r + q + x * PW_LD];
+            aa[q] = bb[q] = cmk(x == r + q ? 1.0 : 0.0, 0.0);
+        }
+#pragma unroll 2
+        for (int m = 0; m < nm; ++m) {
+            const double2 am = S->aP[m * PW_LS + x], bm = S->bP[m * PW_LS + x], lm = S->al[m * PW_LS + x], em = S->be[m * PW_LS + x];
+#pragma unroll
+            for (int q = 0; q < B; ++q) {
+                const double2 fb = S->bP[m * PW_LS + r + q], fa = S->aP[m * PW_LS + r + q];
+                const double2 nb = cmk(-fb.x, -fb.y), na = cmk(-fa.x, -fa.y);
+                cc[q] = cfma(am, nb, cc[q]);
+                aa[q] = cfma(lm, nb, aa[q]);
+                rr[q] = cfma(na, bm, rr[q]);
+                bb[q] = cfma(na, em, bb[q]);
+            }
+        }
+        __syncwarp();
+        double2 an[B], ln[B];
+        if (B == 2) {
+            an[0] = cfma(cc[0], g11, cmul(cc[B - 1], g21)); an[B - 1] = cfma(cc[0], g12, cmul(cc[B - 1], g22));
+            ln[0] = cfma(aa[0], g11, cmul(aa[B - 1], g21)); ln[B - 1] = cfma(aa[0], g12, cmul(aa[B - 1], g22));
+        } else {
+            an[0] = cmul(cc[0], g11);
+            ln[0] = cmul(aa[0], g11);
+        }
+#pragma unroll
+        for (int q = 0; q < B; ++q) {
+            S->aP[(nm + q) * PW_LS + x] = an[q];
+            S->bP[(nm + q) * PW_LS + x] = rr[q];
+            S->al[(nm + q) * PW_LS + x] = ln[q];
+            S->be[(nm + q) * PW_LS + x] = bb[q];
+            p0 = cfma(cmk(-an[q].x, -an[q].y), rr[q], p0);
+            if (B == 2) {
+                const double2 o = cmk(__shfl_xor_sync(0xffffffffu, rr[q].x, 1), __shfl_xor_sync(0xffffffffu, rr[q].y, 1));
+                p1 = cfma(cmk(-an[q].x, -an[q].y), o, p1);
+            }
+        }
+        nm += B;
+        pc = kf + 1;
+        __syncwarp();
+    }
+    // the steps of four accepted rows that Gamma's product takes
+    for (int m = nm; m < ((nm + 3) & ~3); ++m) S->al[m * PW_LS + x] = S->be[m * PW_LS + x] = cmk(0, 0);
+    nties = warp_sum(nties);
+    if (lane == 0) {
+        S->nacc = nm;
+        c.pw_flag[0] = nm > 0;
+        c.stats[ST_PHASE_RE] = ph.x;
+        c.stats[ST_PHASE_IM] = ph.y;
+        c.stats[B == 2 ? ST_ACCV : ST_ACC] += accm;
+        c.stats[ST_NEAR_TIE] += (double)nties;
+        c.stats[B == 2 ? ST_PROPV : ST_PROP] += (double)nu;
+    }
+}
+
 // visit: slices already updated in this half sweep; dir 0 = 0b (bond families
 // 1..nn_nf, then sites), 1 = b0 (sites, then families nn_nf..1) fixes where
 // this call's draws sit in the half sweep's random words; rnd_off >= 0
-// overrides that offset.  last = 1 on the family's last window (statistics).
+// overrides that offset.  The products around the walk are too small for the
+// general GEMM's tiles (32 x 32 and 32 x ne): their k range (F) or columns (Vt)
+// are split over the eight warps, with fragments read from global memory.
 __global__ void __launch_bounds__(256) k_pwin_seq(const ChainDev* __restrict__ chains, int nt, int nf, int w, int visit,
                                                   int dir, int rnd_off) {
     extern __shared__ double2 ssm[];
@@ -314,10 +452,9 @@ __global__ void __launch_bounds__(256) k_pwin_seq(const ChainDev* __restrict__ c
         if (tid == 0) c.pw_flag[0] = 0;
         return;
     }
-    double2* buf = ssm;
-    PUpdSmem* S = (PUpdSmem*)(ssm + ZT_SMEM_ELEMS);
-    const int bond = p.bond, b = p.b, nu = p.nu, nr = p.nr, u0 = p.u0;
-    const int lc = bond ? 2 : md.lcomp;
+    PUpdSmem* S = (PUpdSmem*)ssm;
+    const int bond = p.bond, nr = p.nr, u0 = p.u0;
+    const int lane = tid & 31, warp = tid >> 5, q4 = lane & 3, l4 = lane >> 2;
     if (rnd_off < 0) {
         const int vw = md.lwrapv ? 2 * md.nn_lf * md.nn_nf : 0, uw = md.lwrapu ? 2 * N : 0;
         int within;
@@ -330,181 +467,109 @@ __global__ void __launch_bounds__(256) k_pwin_seq(const ChainDev* __restrict__ c
     double2 *Rg, *Fg, *Gg, *Ut, *Vt;
     pw_ptrs(c, p.R, Rg, Fg, Gg, Ut, Vt);
     for (int x = tid; x < nr; x += nth) S->rows[x] = p.rows ? p.rows[x] : u0 + x;
-    if (tid == 0) {
-        S->phase = cmk(c.stats[ST_PHASE_RE], c.stats[ST_PHASE_IM]);
-        S->accm = 0.0;
-        S->nties = 0.0;
-        S->nacc = 0;
-    }
-    {   // F = Rg UL(:,rows) = Rg ULT(rows,:)^T
-        ZGemmArgs g;
-        g.M = nr; g.N = nr; g.K = ne; g.alpha = cmk(1, 0); g.beta = cmk(0, 0);
-        g.A = Rg; g.lda = nr; g.opA = OP_N;
-        g.B = p.rows ? c.ULT : c.ULT + u0; g.ldb = N; g.opB = OP_T; g.brow = p.rows;
-        g.C = Fg; g.ldc = nr;
-        zgemm_fit(g, buf);
-    }
-    for (int e = tid; e < nr * nr; e += nth) {
-        int x = e % nr, y = e / nr;
-        double2 v = Fg[e];
-        S->F[x + y * PW_LD] = v;
-        S->Pc[x + y * PW_LD] = v;
-        S->Gm[x + y * PW_LD] = cmk(0, 0);
-    }
-    for (int x = tid; x < nr; x += nth) { S->dl[x] = cmk(0, 0); S->accr[x] = 0; }
-    for (int k = tid; k < nu; k += nth) {
-        const int u = u0 + k;
-        const int is = cf[u];
-        const double r1 = u32_stream(rnd[2 * u]);
-        const int iflip = (int)ceil(r1 * (lc - 1));
-        S->uisp[k] = (is + iflip - 1) % lc + 1;
-        S->ur2[k] = u32_stream(rnd[2 * u + 1]);
-        if (bond) {
-            S->ud1[k] = md.vdp[is - 1];
-            S->ud2[k] = md.vdm[is - 1];
-            S->ukk[k] = 0;
-        } else {
-            const int kk = (is - 1) * (lc - 1) + (iflip - 1);
-            S->ud1[k] = md.delta[kk];
-            S->ud2[k] = cmk(0, 0);
-            S->ukk[k] = kk;
+    __syncthreads();
+    {   // F = Rg UL(:,rows) = Rg ULT(rows,:)^T: warp w the columns 16 (w & 1).. and every fourth k step
+        double cr[4][2][2], ci[4][2][2];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) { cr[i][j][0] = cr[i][j][1] = ci[i][j][0] = ci[i][j][1] = 0.0; }
+        int ry[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int y = 16 * (warp & 1) + 8 * j + l4;
+            ry[j] = y < nr ? S->rows[y] : -1;
+        }
+#pragma unroll 2
+        for (int s = warp >> 1; 4 * s < ne; s += 4) {
+            const int l = 4 * s + q4;
+            double2 va[4], vb[2];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) va[i] = (l < ne && 8 * i + l4 < nr) ? Rg[8 * i + l4 + (size_t)l * nr] : cmk(0, 0);
+#pragma unroll
+            for (int j = 0; j < 2; ++j) vb[j] = (l < ne && ry[j] >= 0) ? c.ULT[MIDX(ry[j], l, N)] : cmk(0, 0);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) zdmma(cr[i][j], ci[i][j], va[i], vb[j]);
+        }
+        // partial products over the walk's vectors: warp w at w * 512, element x + 32 (y mod 16)
+        double2* part = S->aP;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    part[warp * 512 + 8 * i + l4 + 32 * (8 * j + 2 * q4 + h)] = cmk(cr[i][j][h], ci[i][j][h]);
+        __syncthreads();
+        for (int e = tid; e < PW_MAXR * PW_MAXR; e += nth) {
+            const int x = e & 31, y = e >> 5, o = x + 32 * (y & 15), h = y >> 4;
+            double2 v = part[h * 512 + o];
+#pragma unroll
+            for (int q = 1; q < 4; ++q) v = cadd(v, part[(h + 2 * q) * 512 + o]);
+            S->F[x + y * PW_LD] = v;
         }
     }
     __syncthreads();
-    const int warp = tid >> 5;
-    for (int k = 0; k < nu; ++k) {
-        const int r0 = k * b;
-        if (warp == 0) {
-            if (tid == 0) {
-                double2 ratiotot, g11, g12 = cmk(0, 0), g21 = cmk(0, 0), g22 = cmk(0, 0);
-                const double2 d1 = S->ud1[k], d2 = S->ud2[k];
-                if (bond) {
-                    double2 v11 = cadd(cmk(1, 0), cmul(S->Pc[r0 + r0 * PW_LD], d1));
-                    double2 v21 = cmul(S->Pc[r0 + 1 + r0 * PW_LD], d1);
-                    double2 v12 = cmul(S->Pc[r0 + (r0 + 1) * PW_LD], d2);
-                    double2 v22 = cadd(cmk(1, 0), cmul(S->Pc[r0 + 1 + (r0 + 1) * PW_LD], d2));
-                    double2 det = csub(cmul(v11, v22), cmul(v12, v21));
-                    ratiotot = det;
-                    double2 id = cdiv(cmk(1, 0), det);
-                    g11 = cmul(cmul(v22, d1), id);
-                    g12 = cmul(cmul(cmk(-v12.x, -v12.y), d1), id);
-                    g21 = cmul(cmul(cmk(-v21.x, -v21.y), d2), id);
-                    g22 = cmul(cmul(v11, d2), id);
-                } else {
-                    const int kk = S->ukk[k];
-                    double2 ratio1 = cadd(cmk(1, 0), cmul(S->Pc[r0 + r0 * PW_LD], d1));
-                    double2 r = ratio1;
-                    for (int f = 1; f < md.nflr; ++f) r = cmul(r, ratio1);
-                    r = cscale(r, md.gam_ratio[kk]);
-                    ratiotot = cmul(r, md.phase_ratio[kk]);
-                    g11 = cdiv(d1, ratio1);
-                }
-                const double2 ph = S->phase;
-                double ratio_re = cmul(ratiotot, ph).x / ph.x;
-                int acc = fabs(ratio_re) > S->ur2[k];
-                if (fabs(fabs(ratio_re) - S->ur2[k]) < DQ_NEAR_TIE) S->nties += 1.0;
-                if (acc) {
-                    double wgt = sqrt(cmul(ratiotot, cconj(ratiotot)).x);
-                    S->phase = cscale(cmul(ph, ratiotot), 1.0 / wgt);
-                    cf[u0 + k] = S->uisp[k];
-                    S->accm += 1.0;
-                    S->gkk[0] = g11; S->gkk[1] = g21; S->gkk[2] = g12; S->gkk[3] = g22;   // column-major b x b
-                    S->dl[r0] = d1;
-                    S->accr[r0] = 1;
-                    if (bond) { S->dl[r0 + 1] = d2; S->accr[r0 + 1] = 1; }
-                    S->nacc += b;
-                }
-                S->acc_flag[k & 1] = acc;
-            }
-        } else {
-            // warps 1..7, while warp 0 decides: columns / rows r of the current
-            // block and Gamma F_Ar, F_rA Gamma (four partial sums per product)
-            for (int e = tid - 32; e < nr * b; e += nth - 32) {
-                int x = e % nr, cc = e / nr;
-                S->colr[x + cc * PW_MAXR] = S->Pc[x + (r0 + cc) * PW_LD];
-                S->rowr[x + cc * PW_MAXR] = S->Pc[r0 + cc + x * PW_LD];
-                double2 a[4] = {cmk(0, 0), cmk(0, 0), cmk(0, 0), cmk(0, 0)};
-                double2 bb[4] = {cmk(0, 0), cmk(0, 0), cmk(0, 0), cmk(0, 0)};
-                int y = 0;
-                for (; y + 3 < r0; y += 4)
+    if (warp == 0) {
+        if (bond) pwin_walk<2>(S, c, md, rnd, cf, u0, p.nu);
+        else pwin_walk<1>(S, c, md, rnd, cf, u0, p.nu);
+    }
+    __syncthreads();
+    const int nm = S->nacc;
+    if (nm == 0) return;
+    {   // Gamma = al be, tiles w and w + 8
+        const int x = 8 * (warp & 3) + l4, y0 = 8 * (warp >> 2);
+        double cr[2][2] = {{0, 0}, {0, 0}}, ci[2][2] = {{0, 0}, {0, 0}};
+        for (int m = q4; m < ((nm + 3) & ~3); m += 4) {
+            const double2 a = S->al[m * PW_LS + x];
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        a[q] = cfma(S->Gm[x + (y + q) * PW_LD], S->F[y + q + (r0 + cc) * PW_LD], a[q]);
-                        bb[q] = cfma(S->F[r0 + cc + (y + q) * PW_LD], S->Gm[y + q + x * PW_LD], bb[q]);
-                    }
-                for (; y < r0; ++y) {
-                    a[0] = cfma(S->Gm[x + y * PW_LD], S->F[y + (r0 + cc) * PW_LD], a[0]);
-                    bb[0] = cfma(S->F[r0 + cc + y * PW_LD], S->Gm[y + x * PW_LD], bb[0]);
-                }
-                S->ikk[x + cc * PW_MAXR] = cadd(cadd(a[0], a[1]), cadd(a[2], a[3]));
-                S->kik[x + cc * PW_MAXR] = cadd(cadd(bb[0], bb[1]), cadd(bb[2], bb[3]));
-            }
+            for (int t = 0; t < 2; ++t) zdmma(cr[t], ci[t], a, S->be[m * PW_LS + y0 + 16 * t + l4]);
         }
-        __syncthreads();
-        if (!S->acc_flag[k & 1]) continue;
-        for (int e = tid; e < nr * nr; e += nth) {
-            int x = e % nr, y = e / nr;
-            const bool xr = (x >= r0 && x < r0 + b), yr = (y >= r0 && y < r0 + b);
-            if (x < r0 && y < r0) {
-                double2 sacc = cmk(0, 0);
-                for (int pp = 0; pp < b; ++pp)
-                    for (int q = 0; q < b; ++q)
-                        sacc = cfma(cmul(S->ikk[x + pp * PW_MAXR], S->gkk[pp + q * b]), S->kik[y + q * PW_MAXR], sacc);
-                S->Gm[x + y * PW_LD] = cadd(S->Gm[x + y * PW_LD], sacc);
-            } else if (xr && y < r0) {
-                double2 sacc = cmk(0, 0);
-                for (int q = 0; q < b; ++q) sacc = cfma(S->gkk[(x - r0) + q * b], S->kik[y + q * PW_MAXR], sacc);
-                S->Gm[x + y * PW_LD] = cmk(-sacc.x, -sacc.y);
-            } else if (x < r0 && yr) {
-                double2 sacc = cmk(0, 0);
-                for (int pp = 0; pp < b; ++pp) sacc = cfma(S->ikk[x + pp * PW_MAXR], S->gkk[pp + (y - r0) * b], sacc);
-                S->Gm[x + y * PW_LD] = cmk(-sacc.x, -sacc.y);
-            } else if (xr && yr) {
-                S->Gm[x + y * PW_LD] = S->gkk[(x - r0) + (y - r0) * b];
-            } else if (x >= r0 + b && y >= r0 + b) {
-                double2 sacc = cmk(0, 0);
-                for (int pp = 0; pp < b; ++pp)
-                    for (int q = 0; q < b; ++q)
-                        sacc = cfma(cmul(S->colr[x + pp * PW_MAXR], S->gkk[pp + q * b]), S->rowr[y + q * PW_MAXR], sacc);
-                S->Pc[x + y * PW_LD] = csub(S->Pc[x + y * PW_LD], sacc);
-            }
-        }
-        __syncthreads();
+#pragma unroll
+        for (int t = 0; t < 2; ++t)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) S->Gm[x + (y0 + 16 * t + 2 * q4 + h) * PW_LS] = cmk(cr[t][h], ci[t][h]);
     }
-    const int any = S->nacc > 0;
-    if (any) {
-        for (int e = tid; e < nr * nr; e += nth) {
-            int x = e % nr, y = e / nr;
-            Gg[e] = S->Gm[x + y * PW_LD];
-        }
-        __syncthreads();
-        ZGemmArgs g;   // Vt = Gamma Rg
-        g.M = nr; g.N = ne; g.K = nr; g.alpha = cmk(1, 0); g.beta = cmk(0, 0);
-        g.A = Gg; g.lda = nr; g.opA = OP_N; g.B = Rg; g.ldb = nr; g.opB = OP_N; g.C = Vt; g.ldc = nr;
-        zgemm_fit(g, buf);
-        for (int e = tid; e < nr * ne; e += nth) {
-            int x = e % nr, l = e / nr;
-            if (S->accr[x]) {
-                double2* q = c.UR + MIDX(S->rows[x], l, N);
-                double2 v = *q;
-                *q = cadd(v, cmul(S->dl[x], v));
+    __syncthreads();
+    // Vt = Gamma Rg, 8 columns of Rg per warp and step
+    for (int l0 = 8 * warp; l0 < ne; l0 += 64) {
+        double cr[4][2], ci[4][2];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { cr[i][0] = cr[i][1] = ci[i][0] = ci[i][1] = 0.0; }
+        double2 vb[8];
+#pragma unroll
+        for (int s = 0; s < 8; ++s)
+            vb[s] = (l0 + l4 < ne && 4 * s + q4 < nr) ? Rg[4 * s + q4 + (size_t)(l0 + l4) * nr] : cmk(0, 0);
+#pragma unroll
+        for (int s = 0; s < 8; ++s)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) zdmma(cr[i], ci[i], S->Gm[8 * i + l4 + (4 * s + q4) * PW_LS], vb[s]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int x = 8 * i + l4, l = l0 + 2 * q4 + h;
+                if (x < nr && l < ne) Vt[x + (size_t)l * nr] = cmk(cr[i][h], ci[i][h]);
             }
-        }
     }
-    if (tid == 0) {
-        c.pw_flag[0] = any;
-        c.stats[ST_PHASE_RE] = S->phase.x;
-        c.stats[ST_PHASE_IM] = S->phase.y;
-        c.stats[bond ? ST_ACCV : ST_ACC] += S->accm;
-        c.stats[ST_NEAR_TIE] += S->nties;
-        c.stats[bond ? ST_PROPV : ST_PROP] += (double)nu;
+    for (int e = tid; e < nr * ne; e += nth) {
+        const int x = e % nr, l = e / nr;
+        const double2 d = S->dl[x];
+        if (d.x != 0.0 || d.y != 0.0) {
+            double2* q = c.UR + MIDX(S->rows[x], l, N);
+            const double2 v = *q;
+            *q = cadd(v, cmul(d, v));
+        }
     }
 }
 
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
-static constexpr size_t PUPD_SMEM = (size_t)ZT_SMEM_ELEMS * sizeof(double2) + sizeof(PUpdSmem) + 64;
+static constexpr size_t PUPD_SMEM = sizeof(PUpdSmem);
+static_assert(offsetof(PUpdSmem, dl) - offsetof(PUpdSmem, aP) >= 8 * 512 * sizeof(double2), "partial products of F");
 static int g_proj_attr = 0;
 
 static void proj_attrs() {
