@@ -1156,6 +1156,7 @@ struct dqmc_handle {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     double last_ms = 0.0;
     int ctas_per_chain = 1;
+    int max_nb = 0;           // most bonds (over all families) of a model
     int max_lq = 0;           // largest number of unit cells over the models
     size_t graph_nodes = 0;
     int proj = 0;
@@ -1290,6 +1291,7 @@ extern "C" int dqmc_gpu_create(const dqmc_params* params, int n_params, int n_ch
         h->nnf_max = std::max(h->nnf_max, m->nn_nf);
         h->maxNe = std::max(h->maxNe, m->p.ne);
         h->max_lq = std::max(h->max_lq, m->lq);
+        h->max_nb = std::max(h->max_nb, m->nn_nf * m->nn_lf);
         h->max_nublock = std::max(h->max_nublock, m->nublock_dev);
     }
     {
@@ -1526,6 +1528,8 @@ static int launch_prog(dqmc_handle* h, int mat_id, const PropProg& prog, int rig
         launch_prop_fft(h->d_chains, h->nch, h->fft_L, h->maxN, mat_id, prog, right, right, 0, h->st);
         return DQMC_OK;
     }
+    PropProg none; none.n = 0;
+    if (!right && !h->fft_L && launch_prop_small(h->d_chains, h->nch, h->maxN, h->max_nb, mat_id, prog, none, h->st)) return DQMC_OK;
     // dense kinetic steps are GEMMs of their own; the element-wise ops between
     // them run as one propagation kernel per stretch
     PropProg seg; seg.n = 0;
@@ -1540,6 +1544,18 @@ static int launch_prog(dqmc_handle* h, int mat_id, const PropProg& prog, int rig
         }
     }
     return DQMC_OK;
+}
+
+// G <- L G R: the two passes of a wrap, in one launch where that applies
+static void launch_wrap(dqmc_handle* h, const PropProg& pl, const PropProg& pr) {
+    if (!h->fft_L && launch_prop_small(h->d_chains, h->nch, h->maxN, h->max_nb, 0 /*G*/, pl, pr, h->st)) {
+        tmark(h, DQMC_PROF_PROP_L);
+        return;
+    }
+    launch_prog(h, 0 /*G*/, pl, 0);
+    tmark(h, DQMC_PROF_PROP_L);
+    launch_prog(h, 0 /*G*/, pr, 1);
+    tmark(h, DQMC_PROF_PROP_R);
 }
 
 // B(nt1, nt2) from the left (Bmat_left_forward, src/dqmc_ft_core.f90:70-121) or
@@ -2094,10 +2110,7 @@ static void enqueue_b0(dqmc_handle* h, int lupdate, int lmeasure) {
         PropProg pl; pl.n = 0; PropProg pr; pr.n = 0;
         prog_k(m, pl, PW_INV, 0);          // left_backward, nf = 1..nnf
         prog_k(m, pr, PW_FWD, 0);          // right_forward, nf = 1..nnf
-        launch_prog(h, MAT_G, pl, 0);
-        tmark(h, DQMC_PROF_PROP_L);
-        launch_prog(h, MAT_G, pr, 1);
-        tmark(h, DQMC_PROF_PROP_R);
+        launch_wrap(h, pl, pr);
         if (lupdate && m.p.rhub != 0.0) { launch_update(h->d_chains, h->nch, h->max_nublock, h->uteam, nt, visit, h->st, 0, 1); tmark(h, DQMC_PROF_UPDATE); }
         pl.n = 0; pr.n = 0;
         prog_v(m, pl, PW_INV, nt);         // u left_backward
@@ -2109,9 +2122,7 @@ static void enqueue_b0(dqmc_handle* h, int lupdate, int lmeasure) {
                 prog_add(pr, PK_VMIX, 0, nf, nt);            // right_forward
                 prog_add(pl, PK_VMIX, 0, nf, nt);            // left_backward
                 if (lupdate) {
-                    launch_prog(h, MAT_G, pl, 0);
-                    launch_prog(h, MAT_G, pr, 1);
-                    tmark(h, DQMC_PROF_PROP_L);
+                    launch_wrap(h, pl, pr);
                     launch_vbond(h, nt, nf, visit, 1);
                     tmark(h, DQMC_PROF_UPDATE);
                     pl.n = 0; pr.n = 0;
@@ -2124,19 +2135,14 @@ static void enqueue_b0(dqmc_handle* h, int lupdate, int lmeasure) {
         if (plq) {
             // the plaquettes (update, then props, descending) between the U field
             // and the kinetic half step (dqmc_ft_sweep_b0.f90:91-101)
-            launch_prog(h, MAT_G, pl, 0);
-            launch_prog(h, MAT_G, pr, 1);
-            tmark(h, DQMC_PROF_PROP_L);
+            launch_wrap(h, pl, pr);
             launch_plq(h, nt, visit, 1, lupdate);
             tmark(h, DQMC_PROF_UPDATE);
             pl.n = 0; pr.n = 0;
         }
         prog_k(m, pl, PW_INV, 1);          // h0 left_backward, nf = nnf..1
         prog_k(m, pr, PW_FWD, 1);
-        launch_prog(h, MAT_G, pl, 0);
-        tmark(h, DQMC_PROF_PROP_L);
-        launch_prog(h, MAT_G, pr, 1);
-        tmark(h, DQMC_PROF_PROP_R);
+        launch_wrap(h, pl, pr);
         if ((m.iwrap_nt[nt - 1] > 0 || m.p.nwrap == 1) || nt == 1) stab_b0(h, m.iwrap_nt[nt - 1]);
     }
 }
@@ -2156,9 +2162,7 @@ static void enqueue_0b(dqmc_handle* h, int lupdate, int lmeasure) {
         if (plq) {
             // the plaquettes (props, then update, ascending) between the kinetic
             // half step and the U field (dqmc_ft_sweep_0b.f90:82-93)
-            launch_prog(h, MAT_G, pl, 0);
-            launch_prog(h, MAT_G, pr, 1);
-            tmark(h, DQMC_PROF_PROP_L);
+            launch_wrap(h, pl, pr);
             launch_plq(h, nt, visit, 0, lupdate);
             tmark(h, DQMC_PROF_UPDATE);
             pl.n = 0; pr.n = 0;
@@ -2172,9 +2176,7 @@ static void enqueue_0b(dqmc_handle* h, int lupdate, int lmeasure) {
                 prog_add(pr, PK_VMIX, 0, nf, nt);            // right_backward
                 prog_add(pr, PK_VSCALE, PW_INV, nf, nt);
                 if (lupdate) {
-                    launch_prog(h, MAT_G, pl, 0);
-                    launch_prog(h, MAT_G, pr, 1);
-                    tmark(h, DQMC_PROF_PROP_L);
+                    launch_wrap(h, pl, pr);
                     launch_vbond(h, nt, nf, visit, 0);
                     tmark(h, DQMC_PROF_UPDATE);
                     pl.n = 0; pr.n = 0;
@@ -2184,18 +2186,12 @@ static void enqueue_0b(dqmc_handle* h, int lupdate, int lmeasure) {
             }
         prog_v(m, pl, PW_FWD, nt);         // u left_forward
         prog_v(m, pr, PW_INV, nt);         // u right_backward
-        launch_prog(h, MAT_G, pl, 0);
-        tmark(h, DQMC_PROF_PROP_L);
-        launch_prog(h, MAT_G, pr, 1);
-        tmark(h, DQMC_PROF_PROP_R);
+        launch_wrap(h, pl, pr);
         if (lupdate && m.p.rhub != 0.0) { launch_update(h->d_chains, h->nch, h->max_nublock, h->uteam, nt, visit, h->st); tmark(h, DQMC_PROF_UPDATE); }
         pl.n = 0; pr.n = 0;
         prog_k(m, pl, PW_FWD, 1);
         prog_k(m, pr, PW_INV, 1);
-        launch_prog(h, MAT_G, pl, 0);
-        tmark(h, DQMC_PROF_PROP_L);
-        launch_prog(h, MAT_G, pr, 1);
-        tmark(h, DQMC_PROF_PROP_R);
+        launch_wrap(h, pl, pr);
         if (lmeasure) { launch_measure_h(h); tmark(h, DQMC_PROF_MEASURE); }
         if (m.iwrap_nt[nt] > 0) stab_0b(h, m.iwrap_nt[nt], 1);
     }
@@ -2245,8 +2241,7 @@ static void enqueue_dyn(dqmc_handle* h) {
         prog_bond(m, pr, PW_INV, nt, 0);
         prog_v(m, pr, PW_INV, nt);
         prog_k(m, pr, PW_INV, 1);
-        launch_prog(h, MAT_G, pl, 0);
-        launch_prog(h, MAT_G, pr, 1);
+        launch_wrap(h, pl, pr);
         if (m.iwrap_nt[nt] > 0) {
             stab_dyn(h, m.iwrap_nt[nt]);
         } else {

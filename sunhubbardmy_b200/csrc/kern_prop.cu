@@ -423,6 +423,147 @@ void launch_prop_fft(const ChainDev* chains, int nchains, int L, int nvec, int m
 #undef PROP_FFT_CASE
 }
 
+// ---------------------------------------------------------------------------
+// Both passes of a slice's wrap, X <- L X R, in one launch for small chains: one CTA
+// holds the whole matrix in shared memory, runs the column program, transposes in
+// place and runs the row program.  At these sizes a pass is latency, not bandwidth: the
+// launch, the pointer chain to the tables and one round trip to the L2 per operator.
+// Here the bond coefficients of every family and the slice's diagonal factors are
+// fetched together, and the matrix is loaded and stored once for both sides.
+// ---------------------------------------------------------------------------
+#define PROP_SMALL_N 64
+
+// element (v, i) of the nv = N vectors at S[v * vs + i]; uf / ui: urt / urtm1 of the bonds, dg: bmat / bmat_inv of the sites
+// of slice nt_diag (other slices' are read where they are used)
+DQ_DEV void small_op(const ModelDev& md, const int32_t* conf, const int32_t* vconf, int code, int right, double2* S,
+                     const double2* uf, const double2* ui, const double2* dg, int nt_diag, const int2* ij) {
+    const int kind = code & 15, which = (code >> 4) & 15, nf = (code >> 8) & 255, nt = code >> 16;
+    const int N = md.N, vs = N + 1, tid = threadIdx.x, nth = blockDim.x;
+    if (kind == PK_DIAG) {
+        const double2* d = dg + (which == PW_INV ? N : 0);
+        const int32_t* cf = conf + (size_t)(nt - 1) * N;
+        const double2* bt = which == PW_INV ? md.bmat_inv : md.bmat;
+        const int ngrp = max(1, min(N, nth / N)), per = (N + ngrp - 1) / ngrp;
+        for (int w = tid; w < N * ngrp; w += nth) {
+            const int i = w % N, v0 = (w / N) * per, v1 = min(N, v0 + per);
+            double2 b = nt == nt_diag ? d[i] : bt[__ldg(&cf[i]) - 1];
+            if (which == PW_CONJ) b.y = -b.y;
+            for (int v = v0; v < v1; ++v) S[v * vs + i] = cmul(S[v * vs + i], b);
+        }
+        __syncthreads();
+        return;
+    }
+    const int lf = md.nn_lf, ngrp = max(1, min(N, nth / lf)), per = (N + ngrp - 1) / ngrp, sp = md.cb_split[nf - 1];
+    const double h = 1.0 / sqrt(2.0);
+    const int32_t* vc = kind == PK_VSCALE ? vconf + ((size_t)(nt - 1) * md.nn_nf + (nf - 1)) * N : nullptr;
+    for (int ph = 0; ph < 2; ++ph) {          // the family's disjoint phases (apply_op)
+        const int b0 = ph ? sp : 0, nbp = ph ? lf - sp : sp;
+        if (ph) {
+            if (nbp == 0) break;
+            __syncthreads();
+        }
+        for (int w = tid; w < nbp * ngrp; w += nth) {
+            const int b = b0 + w % nbp, v0 = (w / nbp) * per, v1 = min(N, v0 + per);
+            const int ist = (nf - 1) * lf + b;
+            const int i1 = ij[ist].x, i2 = ij[ist].y;
+            if (kind == PK_CB) {
+                const double2* u = (which == PW_INV ? ui : uf) + 4 * ist;
+                const double2 c0 = u[0], c1 = u[right ? 2 : 1], c2 = u[right ? 1 : 2], c3 = u[3];
+#pragma unroll 4
+                for (int v = v0; v < v1; ++v) {
+                    double2* x = S + v * vs;
+                    const double2 a = x[i1], c = x[i2];
+                    x[i1] = cadd(cmul(c0, a), cmul(c1, c));
+                    x[i2] = cadd(cmul(c2, a), cmul(c3, c));
+                }
+            } else if (kind == PK_VMIX) {
+                for (int v = v0; v < v1; ++v) {
+                    double2* x = S + v * vs;
+                    const double2 a = x[i1], c = x[i2];
+                    x[i1] = cadd(cscale(a, h), cscale(c, h));
+                    x[i2] = cadd(cscale(a, h), cscale(c, -h));
+                }
+            } else {
+                const int is = __ldg(&vc[b]) - 1;
+                const double2 s1 = (which == PW_INV) ? md.vbpi[is] : md.vbp[is];
+                const double2 s2 = (which == PW_INV) ? md.vbmi[is] : md.vbm[is];
+                for (int v = v0; v < v1; ++v) {
+                    double2* x = S + v * vs;
+                    x[i1] = cmul(s1, x[i1]);
+                    x[i2] = cmul(s2, x[i2]);
+                }
+            }
+        }
+    }
+    __syncthreads();
+}
+
+__global__ void __launch_bounds__(256) k_prop_small(const ChainDev* __restrict__ chains, int mat_id, PropProg pl, PropProg pr,
+                                                    int nt_diag) {
+    extern __shared__ double2 sm[];
+    const ChainDev& c = chains[blockIdx.x];
+    const ModelDev& md = *c.md;
+    const int N = c.N, vs = N + 1, nb = md.nn_nf * md.nn_lf, tid = threadIdx.x, nth = blockDim.x;
+    double2* X = chain_mat(c, mat_id);
+    double2 *S = sm, *uf = S + N * vs, *ui = uf + 4 * nb, *dg = ui + 4 * nb;
+    int2* ij = (int2*)(dg + 2 * N);
+    const int lane = tid & 31, warp = tid >> 5, nw = nth >> 5;
+    for (int j = warp; j < N; j += nw)
+        for (int i = lane; i < N; i += 32) S[j * vs + i] = X[MIDX(i, j, N)];
+    for (int e = tid; e < 4 * nb; e += nth) { uf[e] = __ldg(&md.urt[e]); ui[e] = __ldg(&md.urtm1[e]); }
+    for (int e = tid; e < nb; e += nth) ij[e] = make_int2(__ldg(&md.bond_i1[e]), __ldg(&md.bond_i2[e]));
+    if (nt_diag > 0)
+        for (int i = tid; i < N; i += nth) {
+            const int is = c.conf[(size_t)(nt_diag - 1) * N + i] - 1;
+            dg[i] = md.bmat[is];
+            dg[N + i] = md.bmat_inv[is];
+        }
+    __syncthreads();
+    for (int k = 0; k < pl.n; ++k) small_op(md, c.conf, c.vconf, pl.op[k], 0, S, uf, ui, dg, nt_diag, ij);
+    auto transpose = [&]() {
+        for (int j = warp; j < N; j += nw)
+            for (int i = lane; i < j; i += 32) {
+                const double2 t = S[j * vs + i];
+                S[j * vs + i] = S[i * vs + j];
+                S[i * vs + j] = t;
+            }
+        __syncthreads();
+    };
+    if (pr.n) {
+        transpose();
+        for (int k = 0; k < pr.n; ++k) small_op(md, c.conf, c.vconf, pr.op[k], 1, S, uf, ui, dg, nt_diag, ij);
+        transpose();
+    }
+    for (int j = warp; j < N; j += nw)
+        for (int i = lane; i < N; i += 32) X[MIDX(i, j, N)] = S[j * vs + i];
+}
+
+// L X R in one launch where the chains are small and the programs hold bond and
+// diagonal operators only; returns 0 without launching otherwise.  Two launches of the
+// general passes take 2 x 9 us for 16 sites, and their B product of ten slices 88 us; a
+// chain of more than 64 sites would keep one SM busy longer than its columns spread over several.
+int launch_prop_small(const ChainDev* chains, int nchains, int maxN, int max_nb, int mat_id, const PropProg& pl, const PropProg& pr,
+                      cudaStream_t st) {
+    if (maxN > PROP_SMALL_N || pl.n + pr.n == 0) return 0;
+    int nt = 0;                // the first diagonal operator's slice
+    for (int side = 0; side < 2; ++side) {
+        const PropProg& p = side ? pr : pl;
+        for (int k = 0; k < p.n; ++k) {
+            const int kind = p.op[k] & 15;
+            if (kind != PK_CB && kind != PK_DIAG && kind != PK_VMIX && kind != PK_VSCALE) return 0;
+            if (kind == PK_DIAG && !nt) nt = p.op[k] >> 16;
+        }
+    }
+    const size_t smem = ((size_t)maxN * (maxN + 1) + 8 * (size_t)max_nb + 2 * maxN) * sizeof(double2) + (size_t)max_nb * sizeof(int2);
+    static int attr = 0;
+    if (!attr) {
+        cudaFuncSetAttribute(k_prop_small, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        attr = 1;
+    }
+    k_prop_small<<<nchains, 256, smem, st>>>(chains, mat_id, pl, pr, nt);
+    return 1;
+}
+
 static int g_prop_smem_ok = 0;
 
 void launch_prop(const ChainDev* chains, int nchains, int maxN, int mat_id, const PropProg& prog,

@@ -12,6 +12,10 @@ void launch_prop(const ChainDev* chains, int nchains, int maxN, int mat_id, cons
 int prop_fft_eligible(const PropProg& prog);
 void launch_prop_fft(const ChainDev* chains, int nchains, int L, int nvec, int mat_id, const PropProg& prog,
                      int rows, int right, int tall, cudaStream_t st);
+// X <- L X R of both programs in one launch, for small chains (max_nb: most bonds of a
+// model, over its families); returns 0 without launching where it does not apply
+int launch_prop_small(const ChainDev* chains, int nchains, int maxN, int max_nb, int mat_id, const PropProg& pl, const PropProg& pr,
+                      cudaStream_t st);
 void launch_sfmt(const ChainDev* chains, int nchains, int slices, cudaStream_t st);
 void launch_sfmt_raw(const ChainDev* chains, int chain, int count, cudaStream_t st);
 // dir: the sweep direction of the slice's draws (0: 0b, 1: b0; ModelDev::rw_u)
