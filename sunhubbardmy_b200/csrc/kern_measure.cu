@@ -8,9 +8,9 @@
 // zphi = sgn/Re(phase) * phase.  G^T is written first (a tiled transpose), so
 // that every correlation term reads a column of G or of G^T.  Per chain, one
 // CTA sums the single-number energy terms, and CTAs of site bins (cpcm, spsm,
-// nn, pair_onsite) and of bond bins (jj, bb, pair_nn, pair_sn) follow.  Two
-// threads own a bin (distance d, orbitals a, b); they walk the even and the
-// odd unit cells j in order, pairing j with cell i = j + d (imj(i, j) = d, in
+// nn, pair_onsite) and of bond bins (jj, bb, pair_nn, pair_sn) follow.  SPLIT
+// threads own a bin (distance d, orbitals a, b); they walk the unit cells j of a
+// residue mod SPLIT in order, pairing j with cell i = j + d (imj(i, j) = d, in
 // closed form), and their sums are added in a fixed order, so no atomics are
 // needed and the result does not depend on scheduling.  Threads of
 // consecutive d read consecutive rows of the same columns (coalesced).
@@ -22,8 +22,12 @@
 #include "kernels.h"
 
 #define MEAS_NT 256
-#define MEAS_SPLIT 2                       // threads per bin
-#define MEAS_BH (MEAS_NT / MEAS_SPLIT)    // bins per CTA
+// Threads per bin (SPLIT) and so bins per CTA (MEAS_NT / SPLIT): a bin's walk over the
+// cells is a chain of loads from the L2.  Two threads a bin fill the device from about
+// 30 chains on (and four gave nothing at 296); with fewer chains eight keep four times
+// as many SMs busy with walks a quarter as long.
+#define MEAS_SPLIT_MANY 2
+#define MEAS_SPLIT_FEW 8
 
 DQ_DEV double2 gcf(const double2* G, int N, int i, int j) {   // Gc(i,j)
     double2 g = G[MIDX(j, i, N)];
@@ -214,14 +218,16 @@ DQ_DEV void meas_energy(const ChainDev& c, double2 zphi, double sgn) {
     }
 }
 
-// The cells of a bin are split by residue mod MEAS_SPLIT between threads
-// t + k MEAS_BH of the CTA; the partial sums are added to thread t's in the
+// The cells of a bin are split by residue mod SPLIT between threads
+// t + k MEAS_NT / SPLIT of the CTA; the partial sums are added to thread t's in the
 // order k = 1, 2, ..., so the result does not depend on scheduling.
+template <int SPLIT>
 DQ_DEV void meas_combine(double2& a0, double2& a1, double2& a2, double2& a3, int h) {
-    __shared__ double2 part[4][MEAS_BH];
-    const int t = threadIdx.x % MEAS_BH;
-#pragma unroll
-    for (int k = 1; k < MEAS_SPLIT; ++k) {
+    constexpr int BH = MEAS_NT / SPLIT;
+    __shared__ double2 part[4][BH];
+    const int t = threadIdx.x % BH;
+#pragma unroll 1
+    for (int k = 1; k < SPLIT; ++k) {
         if (h == k) { part[0][t] = a0; part[1][t] = a1; part[2][t] = a2; part[3][t] = a3; }
         __syncthreads();
         if (h == 0) { a0 = cadd(a0, part[0][t]); a1 = cadd(a1, part[1][t]); a2 = cadd(a2, part[2][t]); a3 = cadd(a3, part[3][t]); }
@@ -229,14 +235,14 @@ DQ_DEV void meas_combine(double2& a0, double2& a1, double2& a2, double2& a3, int
     }
 }
 
-// Site-correlation bins (cpcm, spsm, nn, pair_onsite): MEAS_SPLIT threads per
+// Site-correlation bins (cpcm, spsm, nn, pair_onsite): SPLIT threads per
 // bin (distance d, orbitals a, b) walk interleaved cells j in order.  Accumulates
 // S1 = sum GTc, B = sum GTc G, A = sum gcd_i gcd_j, S4 = sum G G with
 // GTc(i, j) = GT(i, j) - delta_ij = -Gc(i, j); whether site i of cell j + d
 // is site j is the same for every cell j (a translation), so it is taken
 // from cell 0.
-template <bool HC, bool D3, bool RC>
-DQ_DEV void meas_site(const ChainDev& c, int bin, double2 zphi) {   // bin of thread t % MEAS_BH
+template <bool HC, bool D3, bool RC, int SPLIT>
+DQ_DEV void meas_site(const ChainDev& c, int bin, double2 zphi) {   // bin of thread t % (MEAS_NT / SPLIT)
     constexpr int NS = HC ? 2 : 1;        // orbital pairs binned separately
     constexpr int NO = RC ? 6 : 1;        // orbitals summed into one bin (r_cubic)
     __shared__ double2 gcd[512];     // Gc(i,i)
@@ -246,7 +252,7 @@ DQ_DEV void meas_site(const ChainDev& c, int bin, double2 zphi) {   // bin of th
     for (int i = threadIdx.x; i < N; i += MEAS_NT) gcd[i] = gcf(G, N, i, i);
     __syncthreads();
     const bool valid = bin < lq * NS * NS;
-    const int h = threadIdx.x / MEAS_BH;      // cells j = h (mod MEAS_SPLIT)
+    const int h = threadIdx.x / (MEAS_NT / SPLIT);      // cells j = h (mod SPLIT)
     if (!valid) bin = 0;
     const double fsp = 1.0 - 1.0 / (double)(nflr * nflr), fn = 1.0 / (double)nflr;
     const int d = bin % lq, ab = bin / lq, a = ab % NS, b = ab / NS;
@@ -256,7 +262,7 @@ DQ_DEV void meas_site(const ChainDev& c, int bin, double2 zphi) {   // bin of th
     if (NO == 1) {
         CellWalk<D3> w(shift, h);
 #pragma unroll 4
-        for (int cj = valid ? h : lq; cj < lq; cj += MEAS_SPLIT, w.step(MEAS_SPLIT)) {
+        for (int cj = valid ? h : lq; cj < lq; cj += SPLIT, w.step(SPLIT)) {
             const int i = w.ci() * NS + a, j = cj * NS + b;
             const size_t o = (size_t)i + (size_t)N * j;
             double2 gtc = GT[o];
@@ -272,7 +278,7 @@ DQ_DEV void meas_site(const ChainDev& c, int bin, double2 zphi) {   // bin of th
         // for d = 0 and oa == ob
         const bool d0 = shift(0) == 0;
         CellWalk<D3> w(shift, h);
-        for (int cj = valid ? h : lq; cj < lq; cj += MEAS_SPLIT, w.step(MEAS_SPLIT)) {
+        for (int cj = valid ? h : lq; cj < lq; cj += SPLIT, w.step(SPLIT)) {
             const int ci = w.ci();
             for (int ob = 0; ob < NO; ++ob) {
                 const int j = cj * NO + ob;
@@ -290,7 +296,7 @@ DQ_DEV void meas_site(const ChainDev& c, int bin, double2 zphi) {   // bin of th
             }
         }
     }
-    meas_combine(s1, sB, sA, s4, h);
+    meas_combine<SPLIT>(s1, sB, sA, s4, h);
     if (!valid || h) return;
     double2* bins = c.bins;
     double2* cpcm = bins + 10;
@@ -304,15 +310,15 @@ DQ_DEV void meas_site(const ChainDev& c, int bin, double2 zphi) {   // bin of th
     if (!D3) pons[k] = cfma(s4, zphi, pons[k]);     // no pair_onsite on the cubic lattice
 }
 
-// Bond-correlation bins (jj, bb, pair_nn, pair_sn): MEAS_SPLIT threads per
+// Bond-correlation bins (jj, bb, pair_nn, pair_sn): SPLIT threads per
 // distance d walk interleaved cells j in order, pairing site i0 of cell i = j + d and its
 // partners with site j0 and its partners.  The partners are translations
 // (current partner pj: nearest neighbour on the square lattice, second
 // neighbour on the honeycomb; bond partner pb: nearest neighbour; pair
 // partner ps: second neighbour), so on the square lattice the Kronecker
 // deltas of Gc = delta - GT depend on d only and are taken from cell 0.
-template <bool HC, bool D3, bool RC>
-DQ_DEV void meas_bond(const ChainDev& c, int d, double2 zphi) {   // distance of thread t % MEAS_BH
+template <bool HC, bool D3, bool RC, int SPLIT>
+DQ_DEV void meas_bond(const ChainDev& c, int d, double2 zphi) {   // distance of thread t % (MEAS_NT / SPLIT)
     constexpr int NS = HC ? 2 : 1;
     __shared__ double2 jcell[512];   // Gc(i0,in) - Gc(in,i0), current partner
     __shared__ double2 bcell[512];   // e Gc(i0,ib) + conj(e) Gc(ib,i0), bond partner
@@ -332,7 +338,7 @@ DQ_DEV void meas_bond(const ChainDev& c, int d, double2 zphi) {   // distance of
     }
     __syncthreads();
     const bool valid = d < lq;
-    const int h = threadIdx.x / MEAS_BH;      // cells j = h (mod MEAS_SPLIT)
+    const int h = threadIdx.x / (MEAS_NT / SPLIT);      // cells j = h (mod SPLIT)
     if (!valid) d = 0;
     const double fn = 1.0 / (double)md.nflr;
     const CellShift<D3> shift(d, md);
@@ -347,7 +353,7 @@ DQ_DEV void meas_bond(const ChainDev& c, int d, double2 zphi) {   // distance of
     double2 sj = cmk(0, 0), sb = cmk(0, 0), sn = cmk(0, 0), ss = cmk(0, 0);
     CellWalk<D3> w(shift, h);
 #pragma unroll 4
-    for (int cj = valid ? h : lq; cj < lq; cj += MEAS_SPLIT, w.step(MEAS_SPLIT)) {
+    for (int cj = valid ? h : lq; cj < lq; cj += SPLIT, w.step(SPLIT)) {
         const int ci = w.ci();
         const int j0 = cj * NS, i0 = ci * NS, jnj = pj[cj], inj = pj[ci];
         const double2 ei = pe[ci], ej = pe[cj];
@@ -402,7 +408,7 @@ DQ_DEV void meas_bond(const ChainDev& c, int d, double2 zphi) {   // distance of
             ss = cfma(g00, gg(ps[ci], ps[cj]), ss);
         }
     }
-    meas_combine(sj, sb, sn, ss, h);
+    meas_combine<SPLIT>(sj, sb, sn, ss, h);
     if (!valid || h) return;
     double2* zjj = c.bins + 10 + 16 * (size_t)lq;
     double2* zbb = zjj + lq;
@@ -417,16 +423,17 @@ DQ_DEV void meas_bond(const ChainDev& c, int d, double2 zphi) {   // distance of
 
 // grid (1 + na + nb, chains): x = 0 the energy terms, then na CTAs of site
 // bins and nb CTAs of bond bins (sized for the largest lattice of the handle)
-template <bool HC, bool D3, bool RC>
+template <bool HC, bool D3, bool RC, int SPLIT>
 __global__ void __launch_bounds__(MEAS_NT, 2) k_measure(const ChainDev* __restrict__ chains, int na) {
     const ChainDev& c = chains[blockIdx.y];
     const double2 phase = cmk(c.stats[ST_PHASE_RE], c.stats[ST_PHASE_IM]);
     const double sgn = phase.x < 0.0 ? -1.0 : 1.0;
     const double2 zphi = cscale(phase, sgn / phase.x);
     const int x = blockIdx.x;
+    constexpr int BH = MEAS_NT / SPLIT;
     if (x == 0) meas_energy(c, zphi, sgn);
-    else if (x <= na) meas_site<HC, D3, RC>(c, (x - 1) * MEAS_BH + threadIdx.x % MEAS_BH, zphi);
-    else meas_bond<HC, D3, RC>(c, (x - 1 - na) * MEAS_BH + threadIdx.x % MEAS_BH, zphi);
+    else if (x <= na) meas_site<HC, D3, RC, SPLIT>(c, (x - 1) * BH + threadIdx.x % BH, zphi);
+    else meas_bond<HC, D3, RC, SPLIT>(c, (x - 1 - na) * BH + threadIdx.x % BH, zphi);
 }
 
 __global__ void k_bins_clear(const ChainDev* __restrict__ chains, int nbins) {
@@ -461,17 +468,24 @@ __global__ void __launch_bounds__(256) k_transpose_g(const ChainDev* __restrict_
     }
 }
 
+template <int SPLIT>
+static void measure_kind(const ChainDev* chains, int nchains, int kind, int maxlq, cudaStream_t st) {
+    constexpr int BH = MEAS_NT / SPLIT;
+    const int ns = kind == MEAS_HONEYCOMB ? 2 : 1;
+    const int na = (maxlq * ns * ns + BH - 1) / BH, nb = (maxlq + BH - 1) / BH;
+    const dim3 grid(1 + na + nb, nchains);
+    if (kind == MEAS_HONEYCOMB) k_measure<true, false, false, SPLIT><<<grid, MEAS_NT, 0, st>>>(chains, na);
+    else if (kind == MEAS_CUBIC) k_measure<false, true, false, SPLIT><<<grid, MEAS_NT, 0, st>>>(chains, na);
+    else if (kind == MEAS_R_CUBIC) k_measure<false, true, true, SPLIT><<<grid, MEAS_NT, 0, st>>>(chains, na);
+    else k_measure<false, false, false, SPLIT><<<grid, MEAS_NT, 0, st>>>(chains, na);
+}
+
 // kind: MEAS_ONE_ORBITAL (square, chain), MEAS_HONEYCOMB, MEAS_CUBIC or MEAS_R_CUBIC
 void launch_measure(const ChainDev* chains, int nchains, int maxN, int kind, int maxlq, cudaStream_t st) {
     const int nt = (maxN + 31) / 32;
     k_transpose_g<<<dim3(nt, nt, nchains), 256, 0, st>>>(chains, MAT_G);
-    const int ns = kind == MEAS_HONEYCOMB ? 2 : 1;
-    const int na = (maxlq * ns * ns + MEAS_BH - 1) / MEAS_BH, nb = (maxlq + MEAS_BH - 1) / MEAS_BH;
-    const dim3 grid(1 + na + nb, nchains);
-    if (kind == MEAS_HONEYCOMB) k_measure<true, false, false><<<grid, MEAS_NT, 0, st>>>(chains, na);
-    else if (kind == MEAS_CUBIC) k_measure<false, true, false><<<grid, MEAS_NT, 0, st>>>(chains, na);
-    else if (kind == MEAS_R_CUBIC) k_measure<false, true, true><<<grid, MEAS_NT, 0, st>>>(chains, na);
-    else k_measure<false, false, false><<<grid, MEAS_NT, 0, st>>>(chains, na);
+    if (nchains <= 16) measure_kind<MEAS_SPLIT_FEW>(chains, nchains, kind, maxlq, st);
+    else measure_kind<MEAS_SPLIT_MANY>(chains, nchains, kind, maxlq, st);
 }
 
 // dyn_measure (src/dqmc_measure/dyn_measure.f90:1-101) at time index nt: the

@@ -1,7 +1,11 @@
 """Paths that the number of chains of a handle selects.
 
 * the bond field's delayed updates on teams of CTAs (a few chains of more than 64
-  sites) and on one CTA per chain: fields and accept counts against the oracle.
+  sites) and on one CTA per chain: fields and accept counts against the oracle;
+* the equal-time measurement with eight and with two threads per bin (up to 16
+  chains, more): the same chain in handles of 1 and of 17 gives the same bins.  A bin
+  sums at most 64 cells of 4 slices per sweep direction in another order, so the two differ by
+  less than 1e-12 of the largest bin.
 """
 import numpy as np
 import pytest
@@ -9,6 +13,13 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 TV = dict(lattice=2, l1=6, l2=6, beta=0.4, dtau=0.1, rv=1.0, nflr=1, kinetic=0, update=1, nwrap=2, nublock=16)
+MEAS = {
+    "square": dict(lattice=1, l1=8, l2=8, kinetic=0),
+    "honeycomb": dict(lattice=2, l1=5, l2=5, kinetic=0),
+    "chain": dict(lattice=3, l1=10, l2=1, kinetic=0),
+    "cubic": dict(lattice=4, l1=4, l2=4, l3=4, kinetic=0),
+    "r_cubic": dict(lattice=5, l1=2, l2=2, l3=2, rtd=0.7, kinetic=0),
+}
 
 
 @pytest.mark.parametrize("n", [1, 6, 40, 160])
@@ -23,3 +34,17 @@ def test_bond_updates(sb, oracle, n):
             assert np.array_equal(g.vconf(c), o.vconf())
             assert g.diag(c)["accepted_v"] == o.diag()["accepted_v"]
             assert np.max(np.abs(g.green(c) - o.green())) < 1e-10
+
+
+@pytest.mark.parametrize("case", list(MEAS))
+def test_measurement(sb, case):
+    kw = dict(beta=0.4, dtau=0.1, rhub=3.0, nflr=2, update=1, hs=1, nwrap=2, nublock=8, **MEAS[case])
+    p = sb.DqmcParams.make(**kw)
+    bins = {}
+    for n in (1, 17):
+        with sb.Dqmc(p, n_chains=n, seeds=[sb.test_seed(c) for c in range(n)]) as g:
+            g.sweep_start()
+            g.obser_init()
+            g.sweeps(1, True)
+            bins[n] = g.bins_raw(0)
+    assert np.max(np.abs(bins[1] - bins[17])) <= 1e-12 * np.max(np.abs(bins[1]))
