@@ -14,61 +14,67 @@
 #define SFMT_N32 624
 #define SFMT_POS1 122
 
-__device__ __forceinline__ void sfmt_recursion(uint32_t* r, const uint32_t* a, const uint32_t* b,
-                                               const uint32_t* cc, const uint32_t* d) {
-    const uint32_t msk[4] = {0xdfffffefU, 0xddfecb7fU, 0xbffaffffU, 0xbffffff6U};
-    // x = a << 8 (128-bit), y = c >> 8 (128-bit)
-    uint64_t ah = ((uint64_t)a[3] << 32) | a[2], al = ((uint64_t)a[1] << 32) | a[0];
-    uint64_t ch = ((uint64_t)cc[3] << 32) | cc[2], cl = ((uint64_t)cc[1] << 32) | cc[0];
-    uint64_t xh = (ah << 8) | (al >> 56), xl = al << 8;
-    uint64_t yh = ch >> 8, yl = (cl >> 8) | (ch << 56);
-    uint32_t x[4] = {(uint32_t)xl, (uint32_t)(xl >> 32), (uint32_t)xh, (uint32_t)(xh >> 32)};
-    uint32_t y[4] = {(uint32_t)yl, (uint32_t)(yl >> 32), (uint32_t)yh, (uint32_t)(yh >> 32)};
-#pragma unroll
-    for (int k = 0; k < 4; ++k) r[k] = a[k] ^ x[k] ^ ((b[k] >> 11) & msk[k]) ^ y[k] ^ (d[k] << 18);
-}
-
-__device__ void sfmt_gen_all(uint32_t* st) {
-    uint32_t* r1 = st + 4 * (SFMT_N - 2);
-    uint32_t* r2 = st + 4 * (SFMT_N - 1);
-    int i;
-    for (i = 0; i < SFMT_N - SFMT_POS1; ++i) {
-        uint32_t out[4];
-        sfmt_recursion(out, st + 4 * i, st + 4 * (i + SFMT_POS1), r1, r2);
-        for (int k = 0; k < 4; ++k) st[4 * i + k] = out[k];
-        r1 = r2; r2 = st + 4 * i;
-    }
-    for (; i < SFMT_N; ++i) {
-        uint32_t out[4];
-        sfmt_recursion(out, st + 4 * i, st + 4 * (i + SFMT_POS1 - SFMT_N), r1, r2);
-        for (int k = 0; k < 4; ++k) st[4 * i + k] = out[k];
-        r1 = r2; r2 = st + 4 * i;
+// The next 156 words of 128 bits, by one warp on the state in shared memory.  Word i
+// is r(i) = t(i) ^ (r(i-2) >> 8) ^ (r(i-1) << 18 per lane), where
+// t(i) = a ^ (a << 8) ^ ((b >> 11) & mask) needs only a = w(i) and b = w(i + 122) of the old
+// state or r(i - 34): the lanes form 32 of the t at once, and the serial part that is
+// left is a few shifts a word, which every lane runs (keeping its own word).  The
+// state is a serial chain of 25,600 words a half sweep for 256 sites and 200 slices.
+__device__ void sfmt_gen_all(uint4* st, uint4* tb) {
+    const int lane = threadIdx.x & 31;
+    uint4 r1 = st[SFMT_N - 2], r2 = st[SFMT_N - 1];
+    for (int i0 = 0; i0 < SFMT_N; i0 += 32) {
+        const int i = i0 + lane, n = min(32, SFMT_N - i0);
+        if (i < SFMT_N) {
+            const uint4 a = st[i], b = st[i + SFMT_POS1 < SFMT_N ? i + SFMT_POS1 : i + SFMT_POS1 - SFMT_N];
+            uint4 t;
+            t.x = a.x ^ (a.x << 8) ^ ((b.x >> 11) & 0xdfffffefU);
+            t.y = a.y ^ __funnelshift_l(a.x, a.y, 8) ^ ((b.y >> 11) & 0xddfecb7fU);
+            t.z = a.z ^ __funnelshift_l(a.y, a.z, 8) ^ ((b.z >> 11) & 0xbffaffffU);
+            t.w = a.w ^ __funnelshift_l(a.z, a.w, 8) ^ ((b.w >> 11) & 0xbffffff6U);
+            tb[lane] = t;
+        }
+        __syncwarp();
+        uint4 mine = make_uint4(0, 0, 0, 0);
+#pragma unroll 4
+        for (int q = 0; q < n; ++q) {
+            uint4 r = tb[q];
+            r.x ^= __funnelshift_r(r1.x, r1.y, 8) ^ (r2.x << 18);
+            r.y ^= __funnelshift_r(r1.y, r1.z, 8) ^ (r2.y << 18);
+            r.z ^= __funnelshift_r(r1.z, r1.w, 8) ^ (r2.z << 18);
+            r.w ^= (r1.w >> 8) ^ (r2.w << 18);
+            r1 = r2;
+            r2 = r;
+            if (q == lane) mine = r;
+        }
+        __syncwarp();
+        if (i < SFMT_N) st[i] = mine;
+        __syncwarp();
     }
 }
 
 // count = slices * rps draws per chain (slices > 0; rps = words per time slice
 // of the chain's model), or exactly -slices draws.  One warp per chain: the
-// state is held in shared memory while lane 0 runs the recursion (the serial
-// part), and the warp copies each block of 624 outputs to the chain's draw
+// state is held in shared memory, and the warp copies each block of 624 outputs to the chain's draw
 // buffer with coalesced stores.
 #define SFMT_WARPS 4
 __global__ void __launch_bounds__(32 * SFMT_WARPS) k_sfmt_fill(const ChainDev* __restrict__ chains, int ch0,
                                                                int nchains, int slices) {
-    __shared__ uint32_t sst[SFMT_WARPS][SFMT_N32];
+    __shared__ uint4 sst[SFMT_WARPS][SFMT_N];
+    __shared__ uint4 stb[SFMT_WARPS][32];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ch = ch0 + blockIdx.x * SFMT_WARPS + w;
     if (ch >= ch0 + nchains) return;      // whole warps; no block barrier below
     const int count = slices > 0 ? slices * chains[ch].md->rps : -slices;
     uint32_t* gst = chains[ch].sfmt;
     uint32_t* out = chains[ch].rnd;
-    uint32_t* s = sst[w];
+    uint32_t* s = (uint32_t*)sst[w];
     for (int e = lane; e < SFMT_N32; e += 32) s[e] = gst[e];
     int idx = (int)gst[SFMT_N32];
     __syncwarp();
     for (int k = 0; k < count;) {
         if (idx >= SFMT_N32) {
-            if (lane == 0) sfmt_gen_all(s);
-            __syncwarp();
+            sfmt_gen_all(sst[w], stb[w]);
             idx = 0;
         }
         const int n = min(SFMT_N32 - idx, count - k);
