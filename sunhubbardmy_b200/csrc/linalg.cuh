@@ -117,9 +117,12 @@ static __device__ void panel_column_careful(double2* P, int m, int ldp, int jb, 
 
 // Householder QR of the m x jb panel, three barriers per column: one pass
 // forms ||P(j+1:m, j)||^2 and the raw products d_c = P(j+1:m, j)^H P(j+1:m, c)
-// together (16-thread groups, one per column), thread 0 forms the reflector
-// and w_c = v^H P(:, c) = P(j, c) + conj(scal) d_c, and one row-owned pass
-// scales the vector and applies P(r, c) -= conj(tau) v_r w_c.
+// together (16-thread groups, one per column), lane 0 of warp 0 forms the reflector
+// and lane c w_c = v^H P(:, c) = P(j, c) + conj(scal) d_c, and one row-owned pass
+// scales the vector and applies P(r, c) -= conj(tau) v_r w_c.  Bound by latency: the
+// loops over rows are unrolled, so that several loads are in flight, and every sum keeps
+// its order.  With it, the unrolled T products and the tiles of apply_block, k_stab /
+// k_green of one 256-site chain take 1.55 / 1.88 ms (1.77 / 2.13 before).
 static __device__ void panel_qr(double2* P, int m, int ldp, int jb, double2* taus, LinalgSmem* L) {
     const int tid = threadIdx.x, nth = blockDim.x;
     const int grp = tid >> 4, gl = tid & 15;
@@ -131,9 +134,11 @@ static __device__ void panel_qr(double2* P, int m, int ldp, int jb, double2* tau
             double2 acc = cmk(0, 0);
             if (ok) {
                 if (g == 0) {
+#pragma unroll 4
                     for (int r = j + 1 + gl; r < m; r += 16) acc.x += cabs2(col[r]);
                 } else {
                     const double2* pc = P + (size_t)(j + g) * ldp;
+#pragma unroll 4
                     for (int r = j + 1 + gl; r < m; r += 16) acc = cfma(cconj(col[r]), pc[r], acc);
                 }
             }
@@ -145,15 +150,17 @@ static __device__ void panel_qr(double2* P, int m, int ldp, int jb, double2* tau
             if (ok && gl == 0) L->w[j + g] = acc;
         }
         __syncthreads();
-        if (tid == 0) {
+        if (tid < 32) {
+            // lane 0 the reflector, then lane cc column cc's w
             const double ss = L->w[j].x;
             const int careful = !(ss < 1e300) || (ss > 0.0 && ss < 1e-280);
-            L->flag = careful;
-            if (!careful) {
-                panel_reflector(col, j, sqrt(ss), taus, L);
-                const double2 cs = cconj(L->scal);
-                for (int cc = j + 1; cc < jb; ++cc) L->w[cc] = cfma(cs, L->w[cc], P[(size_t)cc * ldp + j]);
+            if (tid == 0) {
+                L->flag = careful;
+                if (!careful) panel_reflector(col, j, sqrt(ss), taus, L);
             }
+            __syncwarp();
+            if (!careful && tid > j && tid < jb)
+                L->w[tid] = cfma(cconj(L->scal), L->w[tid], P[(size_t)tid * ldp + j]);
         }
         __syncthreads();
         if (L->flag) {
@@ -166,6 +173,7 @@ static __device__ void panel_qr(double2* P, int m, int ldp, int jb, double2* tau
         for (int r = j + tid; r < m; r += nth) {
             const double2 v = (r == j) ? cmk(1, 0) : cmul(col[r], scal);
             const double2 cv = cmul(ctau, v);
+#pragma unroll 5
             for (int cc = j + 1; cc < jb; ++cc)
                 P[(size_t)cc * ldp + r] = csub(P[(size_t)cc * ldp + r], cmul(cv, L->w[cc]));
             if (r > j) col[r] = v;
@@ -184,6 +192,7 @@ static __device__ void panel_larft(const double2* P, int m, int ldp, int jb, con
         if (a < b) {
             double2 s = P[(size_t)a * ldp + b];          // V(b,a)^* * V(b,b)=1, rows r >= b
             s = cconj(s);
+#pragma unroll 8
             for (int r = b + 1; r < m; ++r) s = cfma(cconj(P[(size_t)a * ldp + r]), P[(size_t)b * ldp + r], s);
             L->S[a + b * QR_NB] = s;
         }
@@ -225,7 +234,9 @@ static __device__ void build_vblock(const double2* A, int N, int p, int jb, doub
     __syncthreads();
 }
 
-// X[p:N, c0:c0+nc] <- (I - V T V^H)^op X,  op = H (apply Q^H) or none (apply Q)
+// X[p:N, c0:c0+nc] <- (I - V T V^H)^op X,  op = H (apply Q^H) or none (apply Q).
+// A team's CTA holds N / size columns (16 of 256): tiles no wider than nc, or most of a
+// 64 x 64 tile (GemmBig) is padding.  The order of each element's sum is the same.
 static __device__ void apply_block(const double2* Vs, const double2* Tp, int N, int p, int jb,
                             double2* X, int c0, int nc, int use_th, LinalgScratch& sc, cplx* gsm) {
     if (nc <= 0) return;
@@ -236,7 +247,8 @@ static __device__ void apply_block(const double2* Vs, const double2* Tp, int N, 
     g.A = Vs; g.lda = N; g.opA = OP_C;
     g.B = X + MIDX(p, c0, N); g.ldb = N; g.opB = OP_N;
     g.C = sc.Ws; g.ldc = QR_NB;
-    zgemm_cta<GemmWide>(g, 0, 1, gsm);
+    if (nc <= 64) zgemm_cta<Gemm16x64>(g, 0, 1, gsm);
+    else zgemm_cta<GemmWide>(g, 0, 1, gsm);
     // W2 = T^H W  or  T W, with T^H or T (16 x 16) in shared memory (the
     // staging buffer is free between the GEMMs); stored as the operator
     // itself, so that threads of consecutive rows a read consecutive elements
@@ -263,7 +275,9 @@ static __device__ void apply_block(const double2* Vs, const double2* Tp, int N, 
     g.A = Vs; g.lda = N; g.opA = OP_N;
     g.B = sc.Ws2; g.ldb = QR_NB; g.opB = OP_N;
     g.C = X + MIDX(p, c0, N); g.ldc = N;
-    zgemm_cta<GemmBig>(g, 0, 1, gsm);
+    if (nc <= 16) zgemm_cta<Gemm64x16>(g, 0, 1, gsm);
+    else if (nc <= 32) zgemm_cta<Gemm64x32>(g, 0, 1, gsm);
+    else zgemm_cta<GemmBig>(g, 0, 1, gsm);
 }
 
 // In-place QR of the first ncol columns of A (N rows, ld N; ncol <= N, default
@@ -456,6 +470,7 @@ static __device__ void build_t64(const double2* Vs, int N, int P, int jb2, const
         for (int e = tid; e < k * jb; e += nth) {
             const int a = e % k, b = e / k;
             double2 acc = cmk(0, 0);
+#pragma unroll 4
             for (int c = a; c < k; ++c) acc = cfma(Tas[a + c * k], Xs[c + b * k], acc);
             Ys[a + b * k] = acc;
         }
@@ -463,6 +478,7 @@ static __device__ void build_t64(const double2* Vs, int N, int P, int jb2, const
         for (int e = tid; e < k * jb; e += nth) {
             const int a = e % k, b = e / k;
             double2 acc = cmk(0, 0);
+#pragma unroll 4
             for (int c = 0; c <= b; ++c) acc = cfma(Ys[a + c * k], Tbs[c + b * QR_NB], acc);
             T64[a + (k + b) * QR_NB2] = cmk(-acc.x, -acc.y);
         }
