@@ -301,8 +301,8 @@ __global__ void __launch_bounds__(256) k_pwin_flush(const ChainDev* __restrict__
 //   a = P(:, r) g, b = P(r, :),  al = (e_r - Gamma F(:, r)) g, be = e_r - F(r, :) Gamma,
 // all four by the same recursion over the m accepted rows (coefficients b_m(r) and
 // a_m(r)), and Gamma = sum_m al_m be_m.  No block barrier inside the walk: with two of
-// them a unit and one thread's divisions it took about 100 of the 171 us that a window of
-// 64 walkers (32 rows, ne = 144) lasted.
+// them a unit and one thread's divisions a family of 64 walkers (288 sites, ne = 144, nine
+// windows of 32 rows, updates included) took 1.54 ms, and 1.31 ms this way.
 template <int B>
 DQ_DEV void pwin_walk(PUpdSmem* S, const ChainDev& c, const ModelDev& md, const uint32_t* rnd, int32_t* cf, int u0, int nu) {
     const int lane = threadIdx.x & 31, k = lane / B, x = lane, lc = B == 2 ? 2 : md.lcomp;
