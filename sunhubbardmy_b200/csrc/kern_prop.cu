@@ -541,7 +541,8 @@ __global__ void __launch_bounds__(256) k_prop_small(const ChainDev* __restrict__
 // L X R in one launch where the chains are small and the programs hold bond and
 // diagonal operators only; returns 0 without launching otherwise.  A wrap of one
 // 16-site chain takes 14.3 + 13.4 us in two launches of the general passes and 15.1 us here
-// (each launch timed by itself), its B product of ten slices 88 against 70 us; a chain of more than 64 sites would keep one SM busy longer than its columns spread over several.
+// (each launch timed by itself), its B product of ten slices 88 against 70 us; a chain
+// of more than 64 sites would keep one SM busy longer than its columns spread over several.
 int launch_prop_small(const ChainDev* chains, int nchains, int maxN, int max_nb, int mat_id, const PropProg& pl, const PropProg& pr,
                       cudaStream_t st) {
     if (maxN > PROP_SMALL_N || pl.n + pr.n == 0) return 0;
