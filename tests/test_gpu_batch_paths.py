@@ -48,3 +48,28 @@ def test_measurement(sb, case):
             g.sweeps(1, True)
             bins[n] = g.bins_raw(0)
     assert np.max(np.abs(bins[1] - bins[17])) <= 1e-12 * np.max(np.abs(bins[1]))
+
+
+# Chains around the 64 sites up to which a wrap is one launch: G of two half sweeps, wraps
+# and B products included, against the oracle (fields equal).
+PROP = {
+    "square64": dict(lattice=1, l1=8, l2=8),
+    "square72": dict(lattice=1, l1=6, l2=12),
+    "honeycomb64": dict(lattice=2, l1=4, l2=8),
+    "chain8": dict(lattice=3, l1=8, l2=1),
+    "cubic64": dict(lattice=4, l1=4, l2=4, l3=4),
+}
+
+
+@pytest.mark.parametrize("case", list(PROP))
+def test_small_chain_propagation(sb, oracle, case):
+    kw = dict(beta=0.6, dtau=0.1, rhub=3.0, mu=0.2, nflr=2, kinetic=0, update=1, hs=1, nwrap=4, nublock=8, **PROP[case])
+    with sb.Dqmc(sb.DqmcParams.make(**kw), n_chains=2, seeds=[sb.test_seed(c) for c in range(2)]) as g:
+        g.sweep_start()
+        g.sweep_b0(); g.sweep_0b()
+        m = oracle.Model(**kw)
+        for c in range(2):
+            o = oracle.Chain(m, sb.test_seed(c))
+            o.sweep_start(); o.sweep_b0(); o.sweep_0b()
+            assert np.array_equal(g.conf(c), o.conf())
+            assert np.max(np.abs(g.green(c) - o.green())) < 1e-10
