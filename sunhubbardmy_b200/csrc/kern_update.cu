@@ -194,7 +194,9 @@ DQ_DEV void upd_extend_rows(const UpdWin* W, const UpdWalk* Y, const double2* G,
 // Every CTA of a team forms the window block and walks it for itself (the same
 // operations on the same values, so the same decisions), which saves an exchange
 // on the serial path; rank 0 alone writes the field and the statistics.  The
-// tiles of steps 3 and 4 are dealt out over the team, which meets after each.
+// tiles of steps 3 and 4 are dealt out over the team, which meets after each, and
+// before a flush that no accepted site of the last window precedes: no CTA
+// stores a tile of G while another may still read its window block from it.
 //
 // forced = 1: the global block move's forced flips of slice nt (sites with
 // blk[i] != 0 go to the next field value, no random test, chains whose block
@@ -368,6 +370,7 @@ __global__ void __launch_bounds__(UPD_NT, 2) k_update_delay(const ChainDev* __re
         __syncthreads();
         // 3. the window's columns on all rows
         const int r = W->r, wend = W->wend;
+        const bool flush = k + r == nb || (w0 + wend >= N && k + r > 0);
         if (r) {
             if (TEAM) {
                 for (int e = tid; e < UPD_L * ((k + 3) & ~3); e += nth) {
@@ -387,12 +390,14 @@ __global__ void __launch_bounds__(UPD_NT, 2) k_update_delay(const ChainDev* __re
             }
             tm.sync();           // the columns are complete; every CTA has read the window's field
             if (tm.rank == 0 && flip) cf[w0 + lane] = nvv;
+        } else if (flush) {
+            tm.sync();           // every CTA has read the window block of G
         } else {
             __syncthreads();
         }
         k += r;
         s = w0 + wend;
-        if (k == nb || (s >= N && k > 0)) {
+        if (flush) {
             flush_addto(G, A, B, N, k, gsm, tm.rank, tm.size);
             tm.sync();
             k = 0;

@@ -61,3 +61,28 @@ def test_sweep(sb, oracle, n):
             assert np.array_equal(g.conf(c), o.conf())
             assert g.diag(c)["accepted"] == o.diag()["accepted"]
             assert np.max(np.abs(g.green(c) - o.green())) < 1e-10
+
+
+@pytest.mark.parametrize("l, n", [(10, 1), (10, 2), (12, 9), (10, 160)])
+def test_forced_flips(sb, l, n):
+    """Block moves of more than 64 sites: most windows of a forced slice hold no
+    forced site, so a slice's flush follows windows that accept nothing.  Local updates off,
+    so the change of the log weight is the sum of the accepted blocks' log ratios
+    (the bounds of test_block_moves_are_exact)."""
+    from sunhubbardmy_b200.learned import EffectiveAction
+    p = sb.DqmcParams.make(lattice=1, l1=l, l2=l, beta=2.0, dtau=0.1, rhub=1.0, nflr=2, kinetic=0, update=1, hs=0,
+                           nwrap=10, nublock=32)
+    nn = EffectiveAction(p.ltrot, l, max_batch=2 * n)
+    nn.set_params(np.zeros(nn.nparams, np.float32))
+    with sb.Dqmc(p, n_chains=n, seeds=[sb.test_seed(c) for c in range(n)]) as g:
+        g.sweep_start()
+        w0 = np.array([g.diag(c)["logweight"].real for c in range(n)])
+        g.reset_diag()
+        g.sweeps_learned(nn, 20, lmeasure=False, seed=77, lupdate=False)
+        for c in range(n):
+            d = g.diag(c)
+            assert d["blk_proposed"] == d["blk_stage1"] > 0
+            assert d["max_wrap_error"] < 1e-8
+            w1 = d["logweight"].real
+            assert abs(p.nflr * (w1 - w0[c]) - d["blk_sum_logratio"]) < 1e-7 * max(1.0, abs(w1))
+        assert sum(g.diag(c)["blk_accepted"] for c in range(n)) > 0
