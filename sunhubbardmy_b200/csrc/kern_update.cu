@@ -438,9 +438,10 @@ __global__ void __launch_bounds__(UPD_NT, 2) k_update_flush(const ChainDev* __re
 // words 2k (iflip) and 2k + 1 (accept test) of the family's draws (0b layout:
 // families ascending after the plaquette words; b0: descending after the U
 // field's).  The rows of the columns and the flush's tiles are dealt out over the
-// chain's team, which meets after each accepted bond; every CTA takes the decisions
-// for itself.  The flush is two thirds of the kernel with one CTA per chain: a family
-// of honeycomb 12 x 12 takes 2.39 ms for 16 chains with one CTA each, 1.22 ms on teams.
+// chain's team, which meets after each accepted bond and before a flush that a
+// rejected one precedes; every CTA takes the decisions for itself.  The flush is two
+// thirds of the kernel with one CTA per chain: a family of honeycomb 12 x 12 takes
+// 2.39 ms for 16 chains with one CTA each, 1.22 ms on teams.
 __global__ void __launch_bounds__(UPD_NT, 2) k_vbond_delay(const ChainDev* __restrict__ chains, int nt, int nf, int visit,
                                                            int dir) {
     extern __shared__ double2 dsm[];                  // flush staging
@@ -507,7 +508,8 @@ __global__ void __launch_bounds__(UPD_NT, 2) k_vbond_delay(const ChainDev* __res
             }
         }
         __syncthreads();
-        if (s_acc) {
+        const bool accepted = s_acc;
+        if (accepted) {
             const int p0 = s_pc[0], p1 = s_pc[1];
             const double2 S00 = s_mat[0], S10 = s_mat[1], S01 = s_mat[2], S11 = s_mat[3];
             for (int i = team.rank * blockDim.x + tid; i < N; i += team.size * blockDim.x) {
@@ -531,6 +533,8 @@ __global__ void __launch_bounds__(UPD_NT, 2) k_vbond_delay(const ChainDev* __res
             if (team.rank == 0 && tid == 0) cf[b] = newval;
         }
         if (k > 0 && (k + 2 > nbv || b == lf - 1)) {
+            // the last bond rejected: every CTA has read G(P,P) before one stores to G
+            if (!accepted) team.sync();
             flush_addto(G, A, B, N, k, dsm, team.rank, team.size);
             team.sync();
             k = 0;

@@ -73,3 +73,22 @@ def test_small_chain_propagation(sb, oracle, case):
             o.sweep_start(); o.sweep_b0(); o.sweep_0b()
             assert np.array_equal(g.conf(c), o.conf())
             assert np.max(np.abs(g.green(c) - o.green())) < 1e-10
+
+
+@pytest.mark.parametrize("n", [1, 6, 40, 160])
+def test_bond_updates_with_rejections(sb, oracle, n):
+    """A strong coupling rejects bonds often, the family's last one among them, so flushes
+    follow rejected bonds; the columns pending then range up to the 64 of a family's flush."""
+    kw = dict(TV, l1=7, l2=6, rv=4.0, nwrap=1, nublock=64)
+    with sb.Dqmc(sb.DqmcParams.make(**kw), n_chains=n, seeds=[sb.test_seed(c) for c in range(n)]) as g:
+        g.sweep_start()
+        g.sweep_b0(); g.sweep_0b()
+        m = oracle.Model(**kw)
+        for c in sorted({0, n - 1}):
+            o = oracle.Chain(m, sb.test_seed(c))
+            o.sweep_start(); o.sweep_b0(); o.sweep_0b()
+            d = g.diag(c)
+            assert d["accepted_v"] < 0.9 * d["proposed_v"]
+            assert np.array_equal(g.vconf(c), o.vconf())
+            assert d["accepted_v"] == o.diag()["accepted_v"]
+            assert np.max(np.abs(g.green(c) - o.green())) < 1e-10
