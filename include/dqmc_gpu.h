@@ -267,6 +267,10 @@ int dqmc_gpu_sweeps_multi(dqmc_handle* const* hs, int nh, int n, int lmeasure, d
 int dqmc_gpu_sweep_start_multi(dqmc_handle* const* hs, int n);
 /* Number of kernel launches in one captured sweep (b0 + 0b) of dqmc_gpu_sweeps. */
 int dqmc_gpu_sweep_kernels(dqmc_handle* h);
+/* CTAs per chain (a thread-block cluster) of the kernels of the last captured sweep of
+ * dqmc_gpu_sweeps, or with multi != 0 of dqmc_gpu_sweeps_multi with several handles; 0
+ * before one.  A handle run beside others takes its share of the device. */
+int dqmc_gpu_sweep_team(dqmc_handle* h, int multi);
 /* Average device time (ms) of `reps` back-to-back launches of one sweep kernel
  * over all chains, timed with CUDA events on the library's stream.  op: 0
  * update of slice 1, 1 UDV stabilisation step, 2 equal-time Green's function,

@@ -1149,10 +1149,12 @@ struct dqmc_handle {
     int nch = 0, maxN = 0, ltrot = 0, nst = 0, nwrap = 0, nnf_max = 0;
     int max_nublock = 1;             // largest flush depth of the models
     int team = 1;                    // CTAs per chain of the QR and Green's function kernels
-    int uteam = 1;                   // and of the update kernel
+    int uteam = 1;                   // and of the update kernels
+    int tiles = 0;                   // site updates extend the delayed columns by tiles (launch_update)
     int started = 0;
-    cudaGraphExec_t sweep_graph = nullptr;
-    int graph_meas = -1;
+    // the captured sweep, [1] with the teams of a run beside other handles
+    cudaGraphExec_t sweep_graph[2] = {nullptr, nullptr};
+    int graph_meas[2] = {-1, -1}, graph_team[2] = {0, 0};
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     double last_ms = 0.0;
     int ctas_per_chain = 1;
@@ -1222,14 +1224,56 @@ static void dfree(dqmc_handle* h, void* p) {
 // the captured sweep holds device pointers and sizes as kernel arguments: any
 // change of them (record buffers) must drop it
 static void drop_sweep_graph(dqmc_handle* h) {
-    if (h->sweep_graph) { cudaGraphExecDestroy(h->sweep_graph); h->sweep_graph = nullptr; }
-    h->graph_meas = -1;
+    for (int s = 0; s < 2; ++s) {
+        if (h->sweep_graph[s]) { cudaGraphExecDestroy(h->sweep_graph[s]); h->sweep_graph[s] = nullptr; }
+        h->graph_meas[s] = -1;
+    }
 }
+
+static void set_team(dqmc_handle* h, int team) {
+    h->team = team;
+    // the update of up to about two windows of sites is its serial walk: 50.6 us a
+    // slice with 4 to 16 CTAs and 52.0 us with one for a chain of 64 sites, 26.9 us
+    // with one and 28.7 us with 8 for 16 sites; at 100 sites 132 us against 192 us
+    h->uteam = h->maxN > 64 ? team : 1;
+}
+
+// CTAs per chain of nh handles that run at once, handle k with nch[k] chains of up to N[k]
+// sites and alone[k] CTAs per chain when it has the device to itself: two CTAs
+// per SM over all handles, dealt out by the chains' sites, and no more than alone[k].
+// Teams that each fill the device queue up behind one another.  Sweeps of 20 slices:
+// 16 handles of 4 chains of 100 sites take 56 ms with 16 CTAs per chain each and 31.6 ms with
+// 2 or 4; 4 handles of 74 chains of 256 sites 189 ms with 2 and 181 ms with one; t-V
+// honeycomb 12 x 12, 8 handles of 8 chains, 199 ms with 8 and 146 ms with 4; honeycomb 6, 9
+// and 12 (48, 48 and 32 chains, four handles each) 103 ms with 8, 8 and 16, 101 ms with 2 for all
+// and 82 ms with 1, 2 and 4.
+static void share_teams(int nh, const int* nch, const int* N, const int* alone, int* team) {
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
+    long long sites = 0;
+    for (int k = 0; k < nh; ++k) sites += (long long)nch[k] * N[k];
+    for (int k = 0; k < nh; ++k)
+        for (team[k] = alone[k]; nh > 1 && team[k] > 1 && team[k] * sites > 2LL * sms * N[k];) team[k] /= 2;
+}
+
+// the handles' shared teams for the lifetime of the object, their own ones after it
+struct SharedTeams {
+    dqmc_handle* const* hs;
+    int n;
+    int own[16];
+    SharedTeams(dqmc_handle* const* hs_, int n_) : hs(hs_), n(n_) {
+        int nch[16], N[16], team[16];
+        for (int k = 0; k < n; ++k) { nch[k] = hs[k]->nch; N[k] = hs[k]->maxN; own[k] = hs[k]->team; }
+        share_teams(n, nch, N, own, team);
+        for (int k = 0; k < n; ++k) set_team(hs[k], team[k]);
+    }
+    ~SharedTeams() { for (int k = 0; k < n; ++k) set_team(hs[k], own[k]); }
+};
 
 extern "C" int dqmc_gpu_destroy(dqmc_handle* h) {
     if (!h) return DQMC_OK;
     if (h->st) cudaStreamSynchronize(h->st);
-    if (h->sweep_graph) cudaGraphExecDestroy(h->sweep_graph);
+    drop_sweep_graph(h);
     for (void* p : h->allocs) cudaFree(p);
     for (HostModel* m : h->models) { for (void* p : m->allocs) cudaFree(p); delete m; }
     if (h->ev0) cudaEventDestroy(h->ev0);
@@ -1456,11 +1500,8 @@ extern "C" int dqmc_gpu_create(const dqmc_params* params, int n_params, int n_ch
         for (int c = 0; c < n_chains; ++c) v[c] = h->chains[c].dev;
         cudaMemcpy(h->d_chains, v.data(), sizeof(ChainDev) * n_chains, cudaMemcpyHostToDevice);
     }
-    h->team = pick_team(n_chains);
-    // the update of up to about two windows of sites is its serial walk: 50.6 us a
-    // slice with 4 to 16 CTAs and 52.0 us with one for a chain of 64 sites, 26.9 us
-    // with one and 28.7 us with 8 for 16 sites; at 100 sites 132 us against 192 us
-    h->uteam = h->maxN > 64 ? h->team : 1;
+    set_team(h, pick_team(n_chains));
+    h->tiles = h->uteam > 1;
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
     h->ctas_per_chain = std::max(1, std::min(h->maxN / 16, (2 * sms + n_chains - 1) / n_chains));
@@ -2050,6 +2091,7 @@ extern "C" int dqmc_gpu_sweep_start_multi(dqmc_handle* const* hs, int n) {
     for (int k = 0; k < n; ++k)
         if (!hs[k]) return fail(DQMC_EINVAL, "null handle");
     int rc0 = DQMC_OK;
+    SharedTeams share(hs, n);
     for (int k = 0; k < n && !rc0; ++k) {
         clear_fail(hs[k]);
         rc0 = sweep_start_impl(hs[k], 0);
@@ -2111,7 +2153,7 @@ static void enqueue_b0(dqmc_handle* h, int lupdate, int lmeasure) {
         prog_k(m, pl, PW_INV, 0);          // left_backward, nf = 1..nnf
         prog_k(m, pr, PW_FWD, 0);          // right_forward, nf = 1..nnf
         launch_wrap(h, pl, pr);
-        if (lupdate && m.p.rhub != 0.0) { launch_update(h->d_chains, h->nch, h->max_nublock, h->uteam, nt, visit, h->st, 0, 1); tmark(h, DQMC_PROF_UPDATE); }
+        if (lupdate && m.p.rhub != 0.0) { launch_update(h->d_chains, h->nch, h->max_nublock, h->uteam, h->tiles, nt, visit, h->st, 0, 1); tmark(h, DQMC_PROF_UPDATE); }
         pl.n = 0; pr.n = 0;
         prog_v(m, pl, PW_INV, nt);         // u left_backward
         prog_v(m, pr, PW_FWD, nt);         // u right_forward
@@ -2187,7 +2229,7 @@ static void enqueue_0b(dqmc_handle* h, int lupdate, int lmeasure) {
         prog_v(m, pl, PW_FWD, nt);         // u left_forward
         prog_v(m, pr, PW_INV, nt);         // u right_backward
         launch_wrap(h, pl, pr);
-        if (lupdate && m.p.rhub != 0.0) { launch_update(h->d_chains, h->nch, h->max_nublock, h->uteam, nt, visit, h->st); tmark(h, DQMC_PROF_UPDATE); }
+        if (lupdate && m.p.rhub != 0.0) { launch_update(h->d_chains, h->nch, h->max_nublock, h->uteam, h->tiles, nt, visit, h->st); tmark(h, DQMC_PROF_UPDATE); }
         pl.n = 0; pr.n = 0;
         prog_k(m, pl, PW_FWD, 1);
         prog_k(m, pr, PW_INV, 1);
@@ -2306,11 +2348,13 @@ extern "C" int dqmc_gpu_sweep_0b(dqmc_handle* h, int lupdate, int lmeasure) {
     return finish_checked(h, 1);
 }
 
-// the captured sweep (b0 + 0b) of dqmc_gpu_sweeps, rebuilt when lmeasure or
-// recording changed
-static int ensure_sweep_graph(dqmc_handle* h, int lmeasure) {
-    if (!h->sweep_graph || h->graph_meas != lmeasure + 2 * h->rec_on) {
-        drop_sweep_graph(h);
+// the captured sweep (b0 + 0b) of dqmc_gpu_sweeps (slot 0) or dqmc_gpu_sweeps_multi (1), rebuilt
+// when lmeasure, recording or the team changed
+static int ensure_sweep_graph(dqmc_handle* h, int slot, int lmeasure) {
+    cudaGraphExec_t& exec = h->sweep_graph[slot];
+    if (!exec || h->graph_meas[slot] != lmeasure + 2 * h->rec_on || h->graph_team[slot] != h->team) {
+        if (exec) { cudaGraphExecDestroy(exec); exec = nullptr; }
+        h->graph_meas[slot] = -1;
         cudaGraph_t g = nullptr;
         CK(cudaStreamBeginCapture(h->st, cudaStreamCaptureModeThreadLocal));
         if (h->proj) {
@@ -2329,16 +2373,17 @@ static int ensure_sweep_graph(dqmc_handle* h, int lmeasure) {
             cudaGetLastError();
             return fail(DQMC_ECUDA, std::string("sweep capture: ") + cudaGetErrorString(e));
         }
-        e = cudaGraphInstantiate(&h->sweep_graph, g, 0);
+        e = cudaGraphInstantiate(&exec, g, 0);
         size_t nn = 0;
         if (e == cudaSuccess) cudaGraphGetNodes(g, nullptr, &nn);
         cudaGraphDestroy(g);
         if (e != cudaSuccess) {
-            h->sweep_graph = nullptr;
+            exec = nullptr;
             return fail(DQMC_ECUDA, std::string("sweep graph instantiation: ") + cudaGetErrorString(e));
         }
         h->graph_nodes = nn;
-        h->graph_meas = lmeasure + 2 * h->rec_on;
+        h->graph_meas[slot] = lmeasure + 2 * h->rec_on;
+        h->graph_team[slot] = h->team;
     }
     return DQMC_OK;
 }
@@ -2347,11 +2392,11 @@ extern "C" int dqmc_gpu_sweeps(dqmc_handle* h, int n, int lmeasure) {
     if (!h) return fail(DQMC_EINVAL, "null handle");
     if (!h->started) return fail(DQMC_ESTATE, "sweep before sweep_start");
     if (n <= 0) return DQMC_OK;
-    int rc = ensure_sweep_graph(h, lmeasure); if (rc) return rc;
+    int rc = ensure_sweep_graph(h, 0, lmeasure); if (rc) return rc;
     h->after_b0 = 0;
     clear_fail(h);
     CK(cudaEventRecord(h->ev0, h->st));
-    for (int i = 0; i < n; ++i) CK(cudaGraphLaunch(h->sweep_graph, h->st));
+    for (int i = 0; i < n; ++i) CK(cudaGraphLaunch(h->sweep_graph[0], h->st));
     CK(cudaEventRecord(h->ev1, h->st));
     CK(cudaStreamSynchronize(h->st));
     CK(cudaGetLastError());
@@ -2375,8 +2420,12 @@ extern "C" int dqmc_gpu_sweeps_multi(dqmc_handle* const* hs, int nh, int n, int 
             if (hs[q] == hs[k]) return fail(DQMC_EINVAL, "a handle appears twice");
     }
     if (n <= 0) return DQMC_OK;
+    const int slot = nh > 1;
+    {
+        SharedTeams share(hs, nh);
+        for (int k = 0; k < nh; ++k) { int rc = ensure_sweep_graph(hs[k], slot, lmeasure); if (rc) return rc; }
+    }
     for (int k = 0; k < nh; ++k) {
-        int rc = ensure_sweep_graph(hs[k], lmeasure); if (rc) return rc;
         hs[k]->after_b0 = 0;
         clear_fail(hs[k]);
     }
@@ -2393,7 +2442,7 @@ extern "C" int dqmc_gpu_sweeps_multi(dqmc_handle* const* hs, int nh, int n, int 
         keep(cudaEventRecord(fork, h0->st));
         for (int k = 1; k < nh; ++k) keep(cudaStreamWaitEvent(hs[k]->st, fork, 0));
         for (int i = 0; i < n && err == cudaSuccess; ++i)
-            for (int k = 0; k < nh; ++k) keep(cudaGraphLaunch(hs[k]->sweep_graph, hs[k]->st));
+            for (int k = 0; k < nh; ++k) keep(cudaGraphLaunch(hs[k]->sweep_graph[slot], hs[k]->st));
         for (int k = 1; k < nh; ++k) {
             keep(cudaEventRecord(join[k], hs[k]->st));
             keep(cudaStreamWaitEvent(h0->st, join[k], 0));
@@ -2418,6 +2467,10 @@ extern "C" int dqmc_gpu_sweeps_multi(dqmc_handle* const* hs, int nh, int n, int 
 extern "C" double dqmc_gpu_last_sweeps_ms(dqmc_handle* h) { return h ? h->last_ms : 0.0; }
 
 extern "C" int dqmc_gpu_sweep_kernels(dqmc_handle* h) { return h ? (int)h->graph_nodes : 0; }
+
+extern "C" int dqmc_gpu_sweep_team(dqmc_handle* h, int multi) {
+    return h && h->sweep_graph[multi != 0] ? h->graph_team[multi != 0] : 0;
+}
 
 // ---------------------------------------------------------------------------
 // data access
@@ -2762,10 +2815,10 @@ extern "C" int dqmc_gpu_update(dqmc_handle* h, int nt) {
         // exactly the 2 N draws of uconf%update (the slice layout of a sweep also
         // holds the plaquette and bond words); the U words start the b0 layout
         launch_sfmt(h->d_chains, h->nch, -2 * m0.N, h->st);
-        launch_update(h->d_chains, h->nch, h->max_nublock, h->uteam, nt, 0, h->st, 0, 1);
+        launch_update(h->d_chains, h->nch, h->max_nublock, h->uteam, h->tiles, nt, 0, h->st, 0, 1);
     } else {
         launch_sfmt(h->d_chains, h->nch, 1, h->st);
-        launch_update(h->d_chains, h->nch, h->max_nublock, h->uteam, nt, 0, h->st);
+        launch_update(h->d_chains, h->nch, h->max_nublock, h->uteam, h->tiles, nt, 0, h->st);
     }
     CK(cudaStreamSynchronize(h->st));
     CK(cudaGetLastError());
@@ -2795,7 +2848,7 @@ extern "C" int dqmc_gpu_time_op(dqmc_handle* h, int op, int reps, double* ms_out
     int spare = h->nst + 1;
     auto enqueue = [&]() {
         switch (op) {
-        case 0: launch_update(h->d_chains, h->nch, h->max_nublock, h->uteam, 1, 0, h->st); break;
+        case 0: launch_update(h->d_chains, h->nch, h->max_nublock, h->uteam, h->tiles, 1, 0, h->st); break;
         case 1: launch_stab_slots(h->d_chains, h->nch, h->maxN, h->team, 0, spare, h->st); break;
         case 2: launch_green(h->d_chains, h->nch, h->maxN, h->team, 1, 0, 0, h->st); break;
         case 3: { PropProg p; p.n = 0; prog_k(m, p, PW_INV, 0); prog_v(m, p, PW_INV, 1); prog_k(m, p, PW_INV, 1);
@@ -3337,7 +3390,7 @@ static int enable_blocks(dqmc_handle* h) {
     for (int c = 0; c < h->nch; ++c) v[c] = h->chains[c].dev;
     CK(copy_sync(h->st, h->d_chains, v.data(), sizeof(ChainDev) * h->nch, cudaMemcpyHostToDevice));
     h->blocks = 1;
-    if (h->sweep_graph) { cudaGraphExecDestroy(h->sweep_graph); h->sweep_graph = nullptr; }
+    drop_sweep_graph(h);
     return DQMC_OK;
 }
 
@@ -3373,7 +3426,7 @@ static void block_move(dqmc_handle* h, dqmc_nn* nn, int t0) {
     launch_nn_forward(nn_w(nn), in, 2 * nch, h->d_S, nullptr, nullptr, h->st);
     launch_blk_begin(h->d_chains, nch, h->d_S, h->d_u, t0, NN_BLK_T, h->st);
     for (int j = 0; j < NN_BLK_T; ++j) {
-        launch_update(h->d_chains, nch, h->max_nublock, h->uteam, t0 + j, 0, h->st, 1);
+        launch_update(h->d_chains, nch, h->max_nublock, h->uteam, h->tiles, t0 + j, 0, h->st, 1);
         if (j + 1 < NN_BLK_T) {
             PropProg pl; pl.n = 0; PropProg pr; pr.n = 0;
             prog_k(m, pl, PW_FWD, 1); prog_k(m, pl, PW_FWD, 0); prog_v(m, pl, PW_FWD, t0 + j + 1);
@@ -3421,7 +3474,7 @@ static void enqueue_0b_blocks(dqmc_handle* h, dqmc_nn* nn, int lupdate, int lmea
         launch_prog(h, MAT_G, pl, 0);
         launch_prog(h, MAT_G, pr, 1);
         if (start[nt]) block_move(h, nn, nt);
-        if (lupdate) launch_update(h->d_chains, h->nch, h->max_nublock, h->uteam, nt, visit, h->st);
+        if (lupdate) launch_update(h->d_chains, h->nch, h->max_nublock, h->uteam, h->tiles, nt, visit, h->st);
         pl.n = 0; pr.n = 0;
         prog_k(m, pl, PW_FWD, 1);
         prog_k(m, pr, PW_INV, 1);

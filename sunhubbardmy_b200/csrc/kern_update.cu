@@ -568,8 +568,10 @@ int launch_vbond_delay(const ChainDev* chains, int nchains, int nublock, int tea
 
 static int g_upd_attr = 0;
 
-void launch_update(const ChainDev* chains, int nchains, int nublock, int team, int nt, int visit, cudaStream_t st, int forced,
-                   int dir) {
+// tiles: the window's columns by upd_extend_tile, else by upd_extend_rows (team 1).  The two differ in
+// rounding, so a handle keeps one of them whatever the team of a run is.
+void launch_update(const ChainDev* chains, int nchains, int nublock, int team, int tiles, int nt, int visit, cudaStream_t st,
+                   int forced, int dir) {
     if (!g_upd_attr) {
         for (const void* k : {(const void*)k_update_delay<false>, (const void*)k_update_delay<true>}) {
             cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, TEAM_SMEM_MAX);
@@ -577,8 +579,8 @@ void launch_update(const ChainDev* chains, int nchains, int nublock, int team, i
         }
         g_upd_attr = 1;
     }
-    launch_team(team > 1 ? k_update_delay<true> : k_update_delay<false>, nchains, team, upd_smem_bytes(nublock, team > 1), st,
-                chains, nt, visit, forced, dir);
+    launch_team(tiles ? k_update_delay<true> : k_update_delay<false>, nchains, team, upd_smem_bytes(nublock, tiles), st, chains,
+                nt, visit, forced, dir);
 }
 
 static int g_flush_attr = 0;

@@ -19,8 +19,8 @@ int launch_prop_small(const ChainDev* chains, int nchains, int maxN, int max_nb,
 void launch_sfmt(const ChainDev* chains, int nchains, int slices, cudaStream_t st);
 void launch_sfmt_raw(const ChainDev* chains, int chain, int count, cudaStream_t st);
 // dir: the sweep direction of the slice's draws (0: 0b, 1: b0; ModelDev::rw_u)
-// nublock: the largest flush depth of the handle's models; team: CTAs per chain
-void launch_update(const ChainDev* chains, int nchains, int nublock, int team, int nt, int visit, cudaStream_t st,
+// nublock: the largest flush depth of the handle's models; team: CTAs per chain (1 without tiles)
+void launch_update(const ChainDev* chains, int nchains, int nublock, int team, int tiles, int nt, int visit, cudaStream_t st,
                    int forced = 0, int dir = 0);
 // one slice of plaquette-field props and updates (dir 0: the 0b order, 1: the b0 order)
 void launch_plq_slice(const ChainDev* chains, int nchains, int maxN, int nt, int visit, int dir, int lupdate,

@@ -151,6 +151,7 @@ SIGNATURES = {
     "dqmc_gpu_last_sweeps_ms": (_d, [_vp]),
     "dqmc_gpu_time_op": (_i, [_vp, _i, _i, _vp]),
     "dqmc_gpu_sweep_kernels": (_i, [_vp]),
+    "dqmc_gpu_sweep_team": (_i, [_vp, _i]),
     "dqmc_gpu_sweep_profile": (_i, [_vp, _i, _i, _vp, _vp]),
     "dqmc_gpu_sweep_dyn": (_i, [_vp]),
     "dqmc_gpu_sweeps_multi": (_i, [_vp, _i, _i, _i, _vp]),
@@ -529,6 +530,11 @@ class Dqmc:
     def sweep_kernels(self) -> int:
         """Kernel launches in one captured sweep (b0 + 0b)."""
         return load_library().dqmc_gpu_sweep_kernels(self.h)
+
+    def sweep_team(self, concurrent: bool = False) -> int:
+        """CTAs per chain in the last captured sweep of `sweeps`, or of
+        `sweeps_concurrent` beside other handles (0 before one)."""
+        return load_library().dqmc_gpu_sweep_team(self.h, int(concurrent))
 
     def time_op(self, op: int, reps: int = 3) -> float:
         """Device ms of one launch of sweep kernel `op` over all chains."""

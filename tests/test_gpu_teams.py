@@ -86,3 +86,43 @@ def test_forced_flips(sb, l, n):
             w1 = d["logweight"].real
             assert abs(p.nflr * (w1 - w0[c]) - d["blk_sum_logratio"]) < 1e-7 * max(1.0, abs(w1))
         assert sum(g.diag(c)["blk_accepted"] for c in range(n)) > 0
+
+
+# sites of a chain and chains of each handle
+GROUPS = {"16x4": [(100, 4)] * 16, "4x20": [(130, 20)] * 4, "2x74": [(98, 74)] * 2, "sizes": [(72, 12), (162, 8), (36, 12)],
+          "2x1": [(130, 1)] * 2}
+
+
+@pytest.mark.parametrize("name", list(GROUPS))
+def test_concurrent_handles_share_the_device(sb, name):
+    """Handles that run at once take two CTAs per SM together, and a handle by itself
+    its own team again; the chains evolve exactly as in separate runs."""
+    import torch
+    slots = 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    runs = []
+    for concurrent in (True, False):
+        hs = [sb.Dqmc(sb.DqmcParams.make(**params(l)), n_chains=n, seeds=[sb.test_seed(100 * k + c) for c in range(n)])
+              for k, (l, n) in enumerate(GROUPS[name])]
+        if concurrent:
+            sb.sweep_start_concurrent(hs)
+            for g in hs:
+                g.obser_init()
+            sb.sweeps_concurrent(hs, 2, True)
+        else:
+            for g in hs:
+                g.sweep_start(); g.obser_init()
+                g.sweeps(2, True)
+        runs.append(hs)
+    a, b = runs
+    shared = [g.sweep_team(True) for g in a]
+    assert all(t >= 1 and t <= g.sweep_team() for t, g in zip(shared, b))
+    assert sum(t * g.n_chains for t, g in zip(shared, a)) <= max(slots, sum(g.n_chains for g in a))
+    for ga, gb in zip(a, b):
+        for c in {0, ga.n_chains - 1}:
+            assert np.array_equal(ga.conf(c), gb.conf(c))
+            assert np.array_equal(ga.green(c), gb.green(c))
+            assert np.array_equal(ga.bins_raw(c), gb.bins_raw(c))
+    a[0].sweeps(1, True)
+    assert a[0].sweep_team() == b[0].sweep_team()
+    for g in a + b:
+        g.close()
