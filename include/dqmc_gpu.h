@@ -271,6 +271,13 @@ int dqmc_gpu_sweep_kernels(dqmc_handle* h);
  * dqmc_gpu_sweeps, or with multi != 0 of dqmc_gpu_sweeps_multi with several handles; 0
  * before one.  A handle run beside others takes its share of the device. */
 int dqmc_gpu_sweep_team(dqmc_handle* h, int multi);
+/* The CTAs per chain (team) that nh handles (1..16) run with at once, handle k with chains[k]
+ * chains of up to sites[k] sites, and whether their site updates extend the delayed columns by
+ * tiles (tiles[k] != 0) or by rows.  dqmc_gpu_set_team gives a handle those of another
+ * run, so that a few chains can be timed with the kernels of many (tune_nublock);
+ * team 1, 2, 4, 8 or 16, rows with team 1 only.  The tiles and the rows differ in rounding. */
+int dqmc_gpu_teams(int nh, const int* chains, const int* sites, int* team, int* tiles);
+int dqmc_gpu_set_team(dqmc_handle* h, int team, int tiles);
 /* Average device time (ms) of `reps` back-to-back launches of one sweep kernel
  * over all chains, timed with CUDA events on the library's stream.  op: 0
  * update of slice 1, 1 UDV stabilisation step, 2 equal-time Green's function,

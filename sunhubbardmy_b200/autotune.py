@@ -25,7 +25,7 @@ import ctypes as C
 
 import numpy as np
 
-from .dqmc import Dqmc, DqmcParams, sweep_start_concurrent, sweeps_concurrent, test_seed
+from .dqmc import Dqmc, DqmcParams, sweep_start_concurrent, sweeps_concurrent, teams, test_seed
 
 
 def with_nublock(p: DqmcParams, nb: int) -> DqmcParams:
@@ -35,11 +35,16 @@ def with_nublock(p: DqmcParams, nb: int) -> DqmcParams:
     return q
 
 
-def tune_nublock(p: DqmcParams, chains: int, candidates=(16, 32, 64), sweeps: int = 1) -> tuple[int, dict]:
-    """Device ms per sweep for each candidate depth on `chains` chains of p."""
+def tune_nublock(p: DqmcParams, chains: int, candidates=(16, 32, 64), sweeps: int = 1, team=None) -> tuple[int, dict]:
+    """Device ms per sweep for each candidate depth on `chains` chains of p, with
+    the kernels of the run that `team` (an entry of dqmc.teams) belongs to:
+    a few chains by themselves take larger teams of CTAs, whose updates cost
+    otherwise."""
     times = {}
     for nb in candidates:
         with Dqmc(with_nublock(p, nb), n_chains=chains) as g:
+            if team:
+                g.set_team(*team)
             g.sweep_start()
             g.sweeps(1, True)                  # captures the sweep graph
             times[nb] = g.sweeps(sweeps, True)
@@ -52,9 +57,11 @@ def batched(groups, tune: bool = True, candidates=(16, 32, 64), tune_chains: int
     Chain order: all chains of the first group, then the second, ...  Seeds are
     the -DTEST formula for consecutive global chain indices."""
     plist, report = [], {}
+    groups = list(groups)
+    team = teams([(sum(n for _, n in groups), max(p.ndim for p, _ in groups))])[0] if tune and groups else None
     for p, n in groups:
         if tune:
-            nb, t = tune_nublock(p, min(n, tune_chains), candidates)
+            nb, t = tune_nublock(p, min(n, tune_chains), candidates, team=team)
             report[p.ndim] = {"nublock": nb, "ms_per_sweep": t}
             p = with_nublock(p, nb)
         plist += [p] * n
@@ -193,13 +200,15 @@ def size_classes(groups, tune: bool = True, candidates=(16, 32, 64), tune_chains
         split = max(1, min(4, ChainGroup.MAX_HANDLES // max(1, len(groups))))
     handles, plist, seeds, report = [], [], [], {}
     c0 = seed0
-    for p, n in groups:
+    parts = [[n // split + (1 if j < n % split else 0) for j in range(min(split, n))] for _, n in groups]
+    runs = [(k, p.ndim) for (p, _), ks in zip(groups, parts) for k in ks]
+    team = teams(runs) if tune and 1 <= len(runs) <= ChainGroup.MAX_HANDLES else None
+    for (p, n), ks in zip(groups, parts):
         if tune:
-            nb, t = tune_nublock(p, min(n, tune_chains), candidates)
+            nb, t = tune_nublock(p, min(n, tune_chains), candidates, team=team[len(handles)] if team and ks else None)
             report[p.ndim] = {"nublock": nb, "ms_per_sweep": t}
             p = with_nublock(p, nb)
-        parts = [n // split + (1 if j < n % split else 0) for j in range(min(split, n))]
-        for k in parts:
+        for k in ks:
             sd = [test_seed(c0 + c) for c in range(k)]
             handles.append(Dqmc(p, n_chains=k, seeds=sd))
             plist += [p] * k

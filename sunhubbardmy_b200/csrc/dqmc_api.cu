@@ -1230,12 +1230,13 @@ static void drop_sweep_graph(dqmc_handle* h) {
     }
 }
 
+// The update of up to about two windows of sites is its serial walk: 50.6 us a
+// slice with 4 to 16 CTAs and 52.0 us with one for a chain of 64 sites, 26.9 us
+// with one and 28.7 us with 8 for 16 sites; at 100 sites 132 us against 192 us.
+static bool use_tiles(int maxN, int team) { return maxN > 64 && team > 1; }
 static void set_team(dqmc_handle* h, int team) {
     h->team = team;
-    // the update of up to about two windows of sites is its serial walk: 50.6 us a
-    // slice with 4 to 16 CTAs and 52.0 us with one for a chain of 64 sites, 26.9 us
-    // with one and 28.7 us with 8 for 16 sites; at 100 sites 132 us against 192 us
-    h->uteam = h->maxN > 64 ? team : 1;
+    h->uteam = use_tiles(h->maxN, team) ? team : 1;
 }
 
 // CTAs per chain of nh handles that run at once, handle k with nch[k] chains of up to N[k]
@@ -1501,7 +1502,7 @@ extern "C" int dqmc_gpu_create(const dqmc_params* params, int n_params, int n_ch
         cudaMemcpy(h->d_chains, v.data(), sizeof(ChainDev) * n_chains, cudaMemcpyHostToDevice);
     }
     set_team(h, pick_team(n_chains));
-    h->tiles = h->uteam > 1;
+    h->tiles = use_tiles(h->maxN, h->team);
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
     h->ctas_per_chain = std::max(1, std::min(h->maxN / 16, (2 * sms + n_chains - 1) / n_chains));
@@ -2470,6 +2471,29 @@ extern "C" int dqmc_gpu_sweep_kernels(dqmc_handle* h) { return h ? (int)h->graph
 
 extern "C" int dqmc_gpu_sweep_team(dqmc_handle* h, int multi) {
     return h && h->sweep_graph[multi != 0] ? h->graph_team[multi != 0] : 0;
+}
+
+extern "C" int dqmc_gpu_teams(int nh, const int* chains, const int* sites, int* team, int* tiles) {
+    if (nh < 1 || nh > 16 || !chains || !sites || !team || !tiles) return fail(DQMC_EINVAL, "1..16 handles");
+    int alone[16];
+    for (int k = 0; k < nh; ++k) {
+        if (chains[k] < 1 || sites[k] < 1) return fail(DQMC_EINVAL, "a handle without chains or sites");
+        alone[k] = pick_team(chains[k]);
+        tiles[k] = use_tiles(sites[k], alone[k]);
+    }
+    share_teams(nh, chains, sites, alone, team);
+    return DQMC_OK;
+}
+
+extern "C" int dqmc_gpu_set_team(dqmc_handle* h, int team, int tiles) {
+    if (!h) return fail(DQMC_EINVAL, "null handle");
+    if (team < 1 || team > 16 || (team & (team - 1))) return fail(DQMC_EINVAL, "team must be 1, 2, 4, 8 or 16");
+    if (!tiles && use_tiles(h->maxN, team)) return fail(DQMC_EINVAL, "a team of several CTAs extends by tiles");
+    CK(cudaStreamSynchronize(h->st));
+    drop_sweep_graph(h);
+    set_team(h, team);
+    h->tiles = tiles != 0;
+    return DQMC_OK;
 }
 
 // ---------------------------------------------------------------------------

@@ -152,6 +152,8 @@ SIGNATURES = {
     "dqmc_gpu_time_op": (_i, [_vp, _i, _i, _vp]),
     "dqmc_gpu_sweep_kernels": (_i, [_vp]),
     "dqmc_gpu_sweep_team": (_i, [_vp, _i]),
+    "dqmc_gpu_teams": (_i, [_i, _vp, _vp, _vp, _vp]),
+    "dqmc_gpu_set_team": (_i, [_vp, _i, _i]),
     "dqmc_gpu_sweep_profile": (_i, [_vp, _i, _i, _vp, _vp]),
     "dqmc_gpu_sweep_dyn": (_i, [_vp]),
     "dqmc_gpu_sweeps_multi": (_i, [_vp, _i, _i, _i, _vp]),
@@ -237,6 +239,15 @@ def qr_logdet_noalloc(n: int, a_dev: int, q_dev: int, logdetq_dev: int, stream: 
                                       C.c_void_p(logdetq_dev), C.c_void_p(stream))
     if rc != 0:
         raise DqmcError(f"qr_logdet_noalloc failed ({rc}): {L.dqmc_gpu_noalloc_error().decode()}")
+
+
+def teams(runs) -> list:
+    """(CTAs per chain, tiles) of handles that run at once, runs = [(chains, sites), ...]
+    (dqmc_gpu_teams)."""
+    n = len(runs)
+    a = [(C.c_int * n)(*v) for v in (*zip(*runs), [0] * n, [0] * n)]
+    _check(load_library().dqmc_gpu_teams(n, *a), "teams")
+    return [(t, bool(s)) for t, s in zip(a[2], a[3])]
 
 
 def sweeps_concurrent(handles, n: int, lmeasure: bool = True) -> float:
@@ -535,6 +546,10 @@ class Dqmc:
         """CTAs per chain in the last captured sweep of `sweeps`, or of
         `sweeps_concurrent` beside other handles (0 before one)."""
         return load_library().dqmc_gpu_sweep_team(self.h, int(concurrent))
+
+    def set_team(self, team: int, tiles: bool) -> None:
+        """Run with the teams of another run (one entry of `teams`)."""
+        _check(load_library().dqmc_gpu_set_team(self.h, int(team), int(tiles)), "set_team")
 
     def time_op(self, op: int, reps: int = 3) -> float:
         """Device ms of one launch of sweep kernel `op` over all chains."""

@@ -126,3 +126,43 @@ def test_concurrent_handles_share_the_device(sb, name):
     assert a[0].sweep_team() == b[0].sweep_team()
     for g in a + b:
         g.close()
+
+
+@pytest.mark.parametrize("n", [40, 160])
+@pytest.mark.parametrize("concurrent", [False, True])
+def test_the_flush_depth_is_timed_with_the_teams_of_the_run(sb, monkeypatch, n, concurrent):
+    """The autotuner times a few chains with the CTAs per chain that the run has."""
+    from sunhubbardmy_b200 import autotune
+    timed = []
+
+    class Timed(sb.Dqmc):
+        def __exit__(self, *a):
+            timed.append(self.sweep_team())
+            return super().__exit__(*a)
+
+    monkeypatch.setattr(autotune, "Dqmc", Timed)
+    build = autotune.size_classes if concurrent else autotune.batched
+    g, _ = build([(sb.DqmcParams.make(**params(98)), n)], candidates=(16, 32))
+    with g:
+        g.sweep_start()
+        g.sweeps(1, True)
+        real = {h.sweep_team(True) for h in g.handles} if concurrent else {g.sweep_team()}
+    assert set(timed[:2]) == real
+
+
+def test_set_team(sb):
+    """Chains of a handle with set teams: the bits of every team above one CTA are the same."""
+    out = []
+    for team in (2, 8, 16):
+        with sb.Dqmc(sb.DqmcParams.make(**params(130)), n_chains=2, seeds=[sb.test_seed(c) for c in range(2)]) as g:
+            g.set_team(team, True)
+            g.sweep_start(); g.obser_init()
+            g.sweeps(2, True)
+            assert g.sweep_team() == team
+            out.append((g.conf(1), g.green(1), g.bins_raw(1)))
+            with pytest.raises(sb.DqmcError):
+                g.set_team(3, True)
+            with pytest.raises(sb.DqmcError):
+                g.set_team(4, False)
+    for a in out[1:]:
+        assert all(np.array_equal(x, y) for x, y in zip(a, out[0]))

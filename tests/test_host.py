@@ -483,3 +483,19 @@ def test_multi_handle_entry_points_check_their_arguments():
     assert L.dqmc_gpu_sweep_start_multi(None, 1) == sb.EINVAL
     assert L.dqmc_gpu_sweep_start_multi(nulls, 2) == sb.EINVAL      # null handles
     assert L.dqmc_gpu_sweeps_multi(nulls, 2, 1, 1, None) == sb.EINVAL
+
+
+def test_team_entry_points_check_their_arguments():
+    """dqmc_gpu_teams refuses an empty or oversized run and handles without chains or
+    sites, dqmc_gpu_set_team a null handle, before any device work."""
+    import ctypes as C
+    import sunhubbardmy_b200 as sb
+    L = sb.load_library()
+    a = [(C.c_int * 17)(*([v] * 17)) for v in (4, 100, 0, 0)]
+    zero = (C.c_int * 17)()
+    for n in (0, 17):
+        assert L.dqmc_gpu_teams(n, *a) == sb.EINVAL
+    assert L.dqmc_gpu_teams(2, zero, *a[1:]) == sb.EINVAL
+    assert L.dqmc_gpu_teams(2, a[0], zero, *a[2:]) == sb.EINVAL
+    assert L.dqmc_gpu_teams(2, a[0], a[1], None, a[3]) == sb.EINVAL
+    assert L.dqmc_gpu_set_team(None, 1, 0) == sb.EINVAL
