@@ -21,6 +21,14 @@
 
 DQ_DEV double u32_to_stream(uint32_t u) { return ((double)u + 0.5) * (1.0 / 4294967296.0); }
 
+// ph times a power of two that brings its larger part near 1 (the quotient of the parts keeps
+// its bits), where it has left 2^-100 .. 2^100
+DQ_DEV double2 near_one(double2 ph) {
+    const int e = max(__double2hiint(ph.x) & 0x7fffffff, __double2hiint(ph.y) & 0x7fffffff) >> 20;
+    if (abs(e - 1023) <= 100 || e == 2047) return ph;
+    return cscale(ph, __hiloint2double((2046 - e) << 20, 0));
+}
+
 // Window of UPD_L consecutive sites, walked by warp 0 (lane p owns site
 // w0 + p).  Its state overlays the GEMM staging buffer, which is only used by
 // the flush after the window has been closed.
@@ -287,8 +295,10 @@ __global__ void __launch_bounds__(UPD_NT, 2) k_update_delay(const ChainDev* __re
             W->pm[lane] = 0;
             __syncwarp();
             // FP64 divides and square roots are dependent chains of 75 to 125 cycles, so
-            // the loop has only delta / ratio: the test multiplies out Re(phase), and the phase, whose modulus the test does not see, is
-            // normalised after the walk (1.7 k cycles per accepted site, 2.3 k before)
+            // the loop has only delta / ratio: the test multiplies out Re(phase), and the
+            // phase, whose modulus the test does not see, is normalised after the walk
+            // (1.7 k cycles per accepted site, 2.3 k before).  Until then near_one keeps it in
+            // range: a flip's ratio may be anything whose square FP64 holds (ratio^nflr).
             int r = 0, pc = 0, wend = L, nties = 0;
             while (pc < L) {
                 const double2 ratio1 = cadd(cmul(csub(cmk(1, 0), dW), dl), cmk(1, 0));
@@ -357,6 +367,7 @@ __global__ void __launch_bounds__(UPD_NT, 2) k_update_delay(const ChainDev* __re
                     Ta[p * UPD_LP + r] = cmul(ta, sscl);
                     Tb[p * UPD_LP + r] = tb;
                 }
+                ph = near_one(ph);
                 ++r;
                 pc = pf + 1;
                 __syncwarp();

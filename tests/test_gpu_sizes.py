@@ -41,3 +41,21 @@ def test_sweeps_at_edge_sizes(sb, oracle, case):
     assert g.diag()["max_wrap_error"] < 1e-9
     bg, bc = g.bins(0), c.bins()
     assert np.max(np.abs(bg["energy"] - bc["energy"])) < 1e-8 * max(1.0, np.max(np.abs(bc["energy"])))
+
+
+@pytest.mark.parametrize("l, u, nflr", [(8, -4.0, 200), (8, 4.0, 100), (10, -4.0, 200), (8, 0.25, 2)])
+def test_many_flavours(sb, oracle, l, u, nflr):
+    """With hundreds of flavours the accepted flips of one window multiply the weight by more
+    than FP64 holds, though each of them (squared) fits: fields and accept counts of the
+    oracle, which normalises the phase after every flip."""
+    kw = dict(lattice=1, l1=l, l2=l, beta=0.4, dtau=0.1, rhub=u, nflr=nflr, kinetic=0, update=1, hs=1, nwrap=2, nublock=64)
+    with sb.Dqmc(sb.DqmcParams.make(**kw), n_chains=2, seeds=[sb.test_seed(c) for c in range(2)]) as g:
+        g.sweep_start()
+        g.sweep_b0(); g.sweep_0b()
+        m = oracle.Model(**kw)
+        for c in range(2):
+            o = oracle.Chain(m, sb.test_seed(c))
+            o.sweep_start(); o.sweep_b0(); o.sweep_0b()
+            assert np.array_equal(g.conf(c), o.conf())
+            assert g.diag(c)["accepted"] == o.diag()["accepted"]
+            assert np.max(np.abs(g.green(c) - o.green())) < 1e-10
