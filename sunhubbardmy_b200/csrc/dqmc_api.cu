@@ -1501,6 +1501,11 @@ extern "C" int dqmc_gpu_create(const dqmc_params* params, int n_params, int n_ch
         for (int c = 0; c < n_chains; ++c) v[c] = h->chains[c].dev;
         cudaMemcpy(h->d_chains, v.data(), sizeof(ChainDev) * n_chains, cudaMemcpyHostToDevice);
     }
+    setup_prop();
+    setup_stab();
+    if (h->proj) setup_proj(); else setup_update();
+    for (const HostModel* m : h->models)
+        if (m->p.rv != 0.0 || m->plq_on) { setup_plq(); break; }
     set_team(h, pick_team(n_chains));
     h->tiles = use_tiles(h->maxN, h->team);
     int sms = 148;
@@ -3145,6 +3150,7 @@ extern "C" int dqmc_nn_create(int ltrot, int l, int max_batch, uint64_t seed, dq
     dqmc_nn* nn = new dqmc_nn();
     nn->Lt = ltrot; nn->L = l; nn->V = ltrot * l * l; nn->maxB = max_batch;
     cudaDeviceGetAttribute(&nn->nsm, cudaDevAttrMultiProcessorCount, 0);
+    setup_nn();
     auto al = [&](size_t bytes) -> void* {
         void* p = nullptr;
         if (cudaMalloc(&p, bytes ? bytes : 16) != cudaSuccess) return nullptr;

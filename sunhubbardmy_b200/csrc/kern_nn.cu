@@ -620,14 +620,11 @@ __global__ void k_nn_pack(const float* theta, bf16* W2T, bf16* W2R) {
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
-static int g_nn_attr = 0;
-static void nn_attrs() {
-    if (g_nn_attr) return;
+void setup_nn() {
     cudaFuncSetAttribute(k_nn_fwd<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)nn_fwd_smem());
     cudaFuncSetAttribute(k_nn_fwd<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)nn_fwd_smem());
     cudaFuncSetAttribute(k_nn_bwd_data, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)nn_bwd_smem());
     cudaFuncSetAttribute(k_nn_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)nn_wgrad_smem());
-    g_nn_attr = 1;
 }
 
 int nn_nbricks(const NNIn& in) {
@@ -635,7 +632,6 @@ int nn_nbricks(const NNIn& in) {
 }
 
 void launch_nn_forward(const NNW& w, const NNIn& in, int B, double* S, bf16* h1g, bf16* h2g, cudaStream_t st) {
-    nn_attrs();
     dim3 grid(nn_nbricks(in), B);
     if (h1g) k_nn_fwd<true><<<grid, 256, nn_fwd_smem(), st>>>(w, in, S, h1g, h2g);
     else k_nn_fwd<false><<<grid, 256, nn_fwd_smem(), st>>>(w, in, S, nullptr, nullptr);
@@ -643,7 +639,6 @@ void launch_nn_forward(const NNW& w, const NNIn& in, int B, double* S, bf16* h1g
 
 void launch_nn_backward(const NNW& w, const NNIn& in, int B, const double* r, const bf16* h1g, const bf16* h2g,
                         bf16* dp2g, float* grad, int nsm, cudaStream_t st) {
-    nn_attrs();
     dim3 grid(nn_nbricks(in), B);
     k_nn_bwd_data<<<grid, 256, nn_bwd_smem(), st>>>(w, in, r, h1g, h2g, dp2g, grad);
     // about two CTAs per SM over the three tap groups; each CTA adds its

@@ -570,21 +570,18 @@ __global__ void __launch_bounds__(PLQ_NT) k_plq_proj_slice(const ChainDev* __res
     }
 }
 
-static int g_plqp_attr = 0;
+void setup_plq() {
+    cudaFuncSetAttribute(k_plq_proj_slice, cudaFuncAttributeMaxDynamicSharedMemorySize, 3 * PLQ_ZMAX * 512 * (int)sizeof(double2));
+    cudaFuncSetAttribute(k_plq_delay, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(k_plq_slice, cudaFuncAttributeMaxDynamicSharedMemorySize, PLQ_ZMAX * 512 * (int)sizeof(double2));
+    cudaFuncSetAttribute(k_vbond_slice, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * 512 * (int)sizeof(double2));
+}
 
 void launch_plq_proj_slice(const ChainDev* chains, int nchains, int maxNe, int nt, int visit, int dir, int lupdate,
                            cudaStream_t st) {
     const size_t smem = (size_t)3 * PLQ_ZMAX * maxNe * sizeof(double2);
-    if (!g_plqp_attr) {
-        cudaFuncSetAttribute(k_plq_proj_slice, cudaFuncAttributeMaxDynamicSharedMemorySize, 3 * PLQ_ZMAX * 512 * (int)sizeof(double2));
-        g_plqp_attr = 1;
-    }
     k_plq_proj_slice<<<nchains, PLQ_NT, smem, st>>>(chains, nt, visit, dir, lupdate);
 }
-
-static int g_plq_attr = 0;
-
-static int g_plqd_attr = 0;
 
 // the delayed plaquette updates when every model's flush depth holds one
 // plaquette's z columns; returns 0 without launching otherwise
@@ -592,10 +589,6 @@ int launch_plq_delay(const ChainDev* chains, int nchains, int nublock, int z, in
                      cudaStream_t st) {
     if (min(nublock, 64) < z) return 0;
     const size_t smem = UpdGemm::SMEM_ELEMS * sizeof(double2);
-    if (!g_plqd_attr) {
-        cudaFuncSetAttribute(k_plq_delay, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        g_plqd_attr = 1;
-    }
     k_plq_delay<<<nchains, PLQ_NT, smem, st>>>(chains, nt, visit, dir);
     return 1;
 }
@@ -603,21 +596,11 @@ int launch_plq_delay(const ChainDev* chains, int nchains, int nublock, int z, in
 void launch_plq_slice(const ChainDev* chains, int nchains, int maxN, int nt, int visit, int dir, int lupdate,
                       cudaStream_t st) {
     const size_t smem = (size_t)PLQ_ZMAX * maxN * sizeof(double2);
-    if (!g_plq_attr) {
-        cudaFuncSetAttribute(k_plq_slice, cudaFuncAttributeMaxDynamicSharedMemorySize, PLQ_ZMAX * 512 * (int)sizeof(double2));
-        g_plq_attr = 1;
-    }
     k_plq_slice<<<nchains, PLQ_NT, smem, st>>>(chains, nt, visit, dir, lupdate);
 }
-
-static int g_vb_attr = 0;
 
 void launch_vbond_slice(const ChainDev* chains, int nchains, int maxN, int nt, int nf, int visit, int dir,
                         cudaStream_t st) {
     const size_t smem = (size_t)2 * maxN * sizeof(double2);
-    if (!g_vb_attr) {
-        cudaFuncSetAttribute(k_vbond_slice, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * 512 * (int)sizeof(double2));
-        g_vb_attr = 1;
-    }
     k_vbond_slice<<<nchains, PLQ_NT, smem, st>>>(chains, nt, nf, visit, dir);
 }

@@ -570,10 +570,8 @@ __global__ void __launch_bounds__(256) k_pwin_seq(const ChainDev* __restrict__ c
 // ---------------------------------------------------------------------------
 static constexpr size_t PUPD_SMEM = sizeof(PUpdSmem);
 static_assert(offsetof(PUpdSmem, dl) - offsetof(PUpdSmem, aP) >= 8 * 512 * sizeof(double2), "partial products of F");
-static int g_proj_attr = 0;
 
-static void proj_attrs() {
-    if (g_proj_attr) return;
+void setup_proj() {
     for (const void* k : {(const void*)k_proj_qr, (const void*)k_proj_ulr}) {
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, TEAM_SMEM_MAX);
         cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -583,22 +581,18 @@ static void proj_attrs() {
     cudaFuncSetAttribute(k_pwin_flush, cudaFuncAttributeMaxDynamicSharedMemorySize, ZT_SMEM_ELEMS * (int)sizeof(double2));
     cudaFuncSetAttribute(k_proj_t1, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmBig::SMEM_ELEMS * (int)sizeof(double2));
     cudaFuncSetAttribute(k_proj_gmat, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmBig::SMEM_ELEMS * (int)sizeof(double2));
-    g_proj_attr = 1;
 }
 
 void launch_proj_qr(const ChainDev* chains, int nchains, int maxN, int team, int mat_id, int dst, int add, cudaStream_t st) {
-    proj_attrs();
     launch_team(k_proj_qr, nchains, team, proj_la_smem(maxN), st, chains, mat_id, dst, add);
 }
 
 void launch_proj_ulr(const ChainDev* chains, int nchains, int maxN, int team, int out_id, int logdet, int ia, int ib, cudaStream_t st) {
-    proj_attrs();
     launch_team(k_proj_ulr, nchains, team, proj_la_smem(maxN), st, chains, out_id, logdet, ia, ib);
 }
 
 void launch_proj_green(const ChainDev* chains, int nchains, int inv_id, int dst_id, int ctas, cudaStream_t st) {
     size_t sm = (size_t)GemmBig::SMEM_ELEMS * sizeof(double2);
-    proj_attrs();
     k_proj_t1<<<dim3(ctas, nchains), 256, sm, st>>>(chains, inv_id);
     k_proj_gmat<<<dim3(ctas, nchains), 256, sm, st>>>(chains, dst_id);
 }
@@ -612,7 +606,6 @@ void launch_tall_copy(const ChainDev* chains, int nchains, int dst_id, int src_i
 void launch_proj_update(const ChainDev* chains, int nchains, int nt, int nf, int visit, int dir, int rnd_off,
                         int nwin, int g_rg, int g_fl, cudaStream_t st) {
     size_t sm = (size_t)ZT_SMEM_ELEMS * sizeof(double2);
-    proj_attrs();
     for (int w = 0; w < nwin; ++w) {
         k_pwin_rg<<<dim3(g_rg, nchains), 256, sm, st>>>(chains, nf, w);
         k_pwin_seq<<<nchains, 256, PUPD_SMEM, st>>>(chains, nt, nf, w, visit, dir, rnd_off);

@@ -556,26 +556,19 @@ int launch_prop_small(const ChainDev* chains, int nchains, int maxN, int max_nb,
         }
     }
     const size_t smem = ((size_t)maxN * (maxN + 1) + 8 * (size_t)max_nb + 2 * maxN) * sizeof(double2) + (size_t)max_nb * sizeof(int2);
-    static int attr = 0;
-    if (!attr) {
-        cudaFuncSetAttribute(k_prop_small, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        attr = 1;
-    }
     k_prop_small<<<nchains, 256, smem, st>>>(chains, mat_id, pl, pr, nt);
     return 1;
 }
 
-static int g_prop_smem_ok = 0;
+void setup_prop() {
+    for (const void* k : {(const void*)k_prop_small, (const void*)k_prop_cols, (const void*)k_prop_rows})
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+}
 
 void launch_prop(const ChainDev* chains, int nchains, int maxN, int mat_id, const PropProg& prog,
                  int right, int ctas_per_chain, cudaStream_t st) {
     const int nb = 16;
     size_t smem = (size_t)nb * (maxN + 1) * sizeof(double2);
-    if (!g_prop_smem_ok) {
-        cudaFuncSetAttribute(k_prop_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        cudaFuncSetAttribute(k_prop_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        g_prop_smem_ok = 1;
-    }
     dim3 grid(ctas_per_chain, nchains);
     if (right) k_prop_rows<<<grid, 256, smem, st>>>(chains, mat_id, prog, nb);
     else k_prop_cols<<<grid, 256, smem, st>>>(chains, mat_id, prog, nb, 0, 0);
@@ -585,11 +578,6 @@ void launch_prop_tall(const ChainDev* chains, int nchains, int maxN, int mat_id,
                       int right, int ctas_per_chain, cudaStream_t st) {
     const int nb = 16;
     size_t smem = (size_t)nb * (maxN + 1) * sizeof(double2);
-    if (!g_prop_smem_ok) {
-        cudaFuncSetAttribute(k_prop_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        cudaFuncSetAttribute(k_prop_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        g_prop_smem_ok = 1;
-    }
     dim3 grid(ctas_per_chain, nchains);
     k_prop_cols<<<grid, 256, smem, st>>>(chains, mat_id, prog, nb, 1, right);
 }

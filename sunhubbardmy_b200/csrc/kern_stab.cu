@@ -564,15 +564,15 @@ __global__ void k_swap_slots(int* slotmap, int n, int spare) {
     }
 }
 
-static int g_stab_attr = 0;
-static void stab_attrs() {
-    if (g_stab_attr) return;
+__global__ void k_kin_dense(const ChainDev* __restrict__ chains, int mat_id, int which, int right, int tall);
+__global__ void k_chain_gemm(const ChainDev* __restrict__ chains, int a_id, int b_id);
+void setup_stab() {
     for (const void* k : {(const void*)k_stab, (const void*)k_green, (const void*)k_green_tau, (const void*)k_qr_test}) {
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, TEAM_SMEM_MAX);
         cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     }
-    cudaFuncSetAttribute(k_zgemm_test, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    g_stab_attr = 1;
+    for (const void* k : {(const void*)k_kin_dense, (const void*)k_chain_gemm, (const void*)k_zgemm_test})
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(GemmBig::SMEM_ELEMS * sizeof(double2)));
 }
 
 // CTAs per chain of the QR and Green's function kernels: the largest cluster of
@@ -582,7 +582,7 @@ static void stab_attrs() {
 // sites take 4.4 ms for 8 chains with 8 CTAs each and 5.2 ms with 16, and 5.4 ms
 // for 16 chains with 4 against 5.9 ms with 8 (10.8 ms with one CTA per chain).
 int pick_team(int nchains) {
-    stab_attrs();
+    setup_stab();
     for (int t = 16; t > 1; t /= 2) {
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute at[1];
@@ -595,17 +595,14 @@ int pick_team(int nchains) {
 }
 
 void launch_stab_slots(const ChainDev* chains, int nchains, int maxN, int team, int src, int dst, cudaStream_t st) {
-    stab_attrs();
     launch_team(k_stab, nchains, team, stab_smem_bytes(maxN), st, chains, src, dst);
 }
 
 void launch_green(const ChainDev* chains, int nchains, int maxN, int team, int nr, int nl, int mode, cudaStream_t st) {
-    stab_attrs();
     launch_team(k_green, nchains, team, stab_smem_bytes(maxN), st, chains, nr, nl, mode);
 }
 
 void launch_green_tau(const ChainDev* chains, int nchains, int maxN, int team, int nr, int nl, cudaStream_t st) {
-    stab_attrs();
     launch_team(k_green_tau, nchains, team, stab_smem_bytes(maxN), st, chains, nr, nl);
 }
 
@@ -707,29 +704,15 @@ __global__ void __launch_bounds__(256) k_dyn_err(const ChainDev* __restrict__ ch
     }
 }
 
-static int g_kin_attr = 0;
-
 void launch_kin_dense(const ChainDev* chains, int nchains, int maxN, int mat_id, int which, int right, int tall,
                       cudaStream_t st) {
-    if (!g_kin_attr) {
-        cudaFuncSetAttribute(k_kin_dense, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(GemmBig::SMEM_ELEMS * sizeof(double2)));
-        g_kin_attr = 1;
-    }
     const int tiles = ((maxN + GemmBig::BM - 1) / GemmBig::BM) * ((maxN + GemmBig::BN - 1) / GemmBig::BN);
     k_kin_dense<<<dim3(tiles, nchains), 256, GemmBig::SMEM_ELEMS * sizeof(double2), st>>>(chains, mat_id, which, right, tall);
     k_kin_copy<<<dim3((maxN * maxN + 255) / 256, nchains), 256, 0, st>>>(chains, mat_id, tall, 0);
 }
 
-static int g_cg_attr = 0;
-
 void launch_chain_gemm(const ChainDev* chains, int nchains, int maxN, int dst_id, int a_id, int b_id, int sub,
                        cudaStream_t st) {
-    if (!g_cg_attr) {
-        cudaFuncSetAttribute(k_chain_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(GemmBig::SMEM_ELEMS * sizeof(double2)));
-        g_cg_attr = 1;
-    }
     const int tiles = ((maxN + GemmBig::BM - 1) / GemmBig::BM) * ((maxN + GemmBig::BN - 1) / GemmBig::BN);
     k_chain_gemm<<<dim3(tiles, nchains), 256, GemmBig::SMEM_ELEMS * sizeof(double2), st>>>(chains, a_id, b_id);
     k_kin_copy<<<dim3((maxN * maxN + 255) / 256, nchains), 256, 0, st>>>(chains, dst_id, 0, sub);
@@ -741,12 +724,10 @@ void launch_dyn_err(const ChainDev* chains, int nchains, cudaStream_t st) {
 
 void launch_zgemm_test(const ChainDev* chains, int nchains, int m, int n, int k, int opa, int opb,
                        int a_id, int b_id, int c_id, double beta_re, cudaStream_t st) {
-    stab_attrs();
     dim3 grid(1, nchains);   // one CTA per chain, as in the stabilisation kernels
     k_zgemm_test<<<grid, 256, GemmBig::SMEM_ELEMS * sizeof(double2), st>>>(chains, m, n, k, opa, opb, a_id, b_id, c_id, beta_re);
 }
 
 void launch_qr_test(const ChainDev* chains, int nchains, int maxN, int team, int a_id, int q_id, cudaStream_t st) {
-    stab_attrs();
     launch_team(k_qr_test, nchains, team, stab_smem_bytes(maxN), st, chains, a_id, q_id);
 }

@@ -560,7 +560,13 @@ __global__ void __launch_bounds__(UPD_NT, 2) k_vbond_delay(const ChainDev* __res
     }
 }
 
-static int g_vbd_attr = 0;
+void setup_update() {
+    for (const void* k : {(const void*)k_update_delay<false>, (const void*)k_update_delay<true>, (const void*)k_vbond_delay}) {
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, TEAM_SMEM_MAX);
+        cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    }
+    cudaFuncSetAttribute(k_update_flush, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+}
 
 // the delayed bond updates when the flush depth allows two columns, else the
 // rank-2 updates straight on G (kern_plqu.cu)
@@ -568,39 +574,19 @@ int launch_vbond_delay(const ChainDev* chains, int nchains, int nublock, int tea
                        cudaStream_t st) {
     if ((min(nublock, 64) & ~1) < 2) return 0;
     const size_t smem = UpdGemm::SMEM_ELEMS * sizeof(double2);
-    if (!g_vbd_attr) {
-        cudaFuncSetAttribute(k_vbond_delay, cudaFuncAttributeMaxDynamicSharedMemorySize, TEAM_SMEM_MAX);
-        cudaFuncSetAttribute(k_vbond_delay, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        g_vbd_attr = 1;
-    }
     launch_team(k_vbond_delay, nchains, team, smem, st, chains, nt, nf, visit, dir);
     return 1;
 }
-
-static int g_upd_attr = 0;
 
 // tiles: the window's columns by upd_extend_tile, else by upd_extend_rows (team 1).  The two differ in
 // rounding, so a handle keeps one of them whatever the team of a run is.
 void launch_update(const ChainDev* chains, int nchains, int nublock, int team, int tiles, int nt, int visit, cudaStream_t st,
                    int forced, int dir) {
-    if (!g_upd_attr) {
-        for (const void* k : {(const void*)k_update_delay<false>, (const void*)k_update_delay<true>}) {
-            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, TEAM_SMEM_MAX);
-            cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        }
-        g_upd_attr = 1;
-    }
     launch_team(tiles ? k_update_delay<true> : k_update_delay<false>, nchains, team, upd_smem_bytes(nublock, tiles), st, chains,
                 nt, visit, forced, dir);
 }
 
-static int g_flush_attr = 0;
-
 void launch_update_flush(const ChainDev* chains, int nchains, cudaStream_t st) {
     size_t smem = UpdGemm::SMEM_ELEMS * sizeof(double2);
-    if (!g_flush_attr) {
-        cudaFuncSetAttribute(k_update_flush, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        g_flush_attr = 1;
-    }
     k_update_flush<<<nchains, UPD_NT, smem, st>>>(chains);
 }

@@ -16,6 +16,13 @@ void launch_prop_fft(const ChainDev* chains, int nchains, int L, int nvec, int m
 // model, over its families); returns 0 without launching where it does not apply
 int launch_prop_small(const ChainDev* chains, int nchains, int maxN, int max_nb, int mat_id, const PropProg& pl, const PropProg& pr,
                       cudaStream_t st);
+// Shared-memory limits and cluster sizes of the kernels, for the current device: set whenever a
+// handle is created, since a device that the process has not used before has the defaults.
+void setup_prop();
+void setup_stab();
+void setup_update();
+void setup_proj();
+void setup_plq();
 void launch_sfmt(const ChainDev* chains, int nchains, int slices, cudaStream_t st);
 void launch_sfmt_raw(const ChainDev* chains, int chain, int count, cudaStream_t st);
 // dir: the sweep direction of the slice's draws (0: 0b, 1: b0; ModelDev::rw_u)

@@ -121,3 +121,15 @@ def test_projective_singular_ulr_returns_enumeric(sb):
     with pytest.raises(sb.DqmcError) as e:
         g.proj_green()
     assert e.value.code == sb.ENUMERIC and g.diag(0)["info"] & sb.FAIL_SINGULAR
+
+
+def test_handles_on_a_device_new_to_the_process():
+    """The kernels' shared-memory limits belong to a device: a handle sets them on its own,
+    whatever the process set elsewhere before (tests/_fresh_device.py)."""
+    import os
+    import subprocess
+    import sys
+    script = os.path.join(os.path.dirname(os.path.abspath(__file__)), "_fresh_device.py")
+    out = subprocess.run([sys.executable, script], capture_output=True, text=True, timeout=300)
+    lines = out.stdout.split("\n")[:-1]
+    assert len(lines) == 9 and all(line.endswith(" True") for line in lines), out.stdout + out.stderr
