@@ -1158,6 +1158,7 @@ struct dqmc_handle {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     double last_ms = 0.0;
     int ctas_per_chain = 1;
+    int spread = 0;           // the general passes hold all columns at once, on SMs of their own
     int max_nb = 0;           // most bonds (over all families) of a model
     int max_lq = 0;           // largest number of unit cells over the models
     size_t graph_nodes = 0;
@@ -1511,6 +1512,13 @@ extern "C" int dqmc_gpu_create(const dqmc_params* params, int n_params, int n_ch
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
     h->ctas_per_chain = std::max(1, std::min(h->maxN / 16, (2 * sms + n_chains - 1) / n_chains));
+    // Where the general passes' CTAs, 16 columns each, hold every chain's columns in one round, k_prop_small
+    // has no more than the second pass's launch to save: B products (one pass) and wraps
+    // by long programs are left to them.  Ten slices' B product, there and in k_prop_small: square 8 x 8
+    // 110 and 133 us for 1 chain, cubic 4^3 160 and 236; 16 sites (one CTA) 89 and 70, 8 x 8 with 148
+    // chains 272 and 141.  A sweep of ten slices, wraps by general passes and by k_prop_small: cubic 4^3
+    // (six families) 3.76 and 3.98 ms, 8 x 8 (four) 3.52 and 3.50 ms.
+    h->spread = h->maxN > 32 && 16 * h->ctas_per_chain >= h->maxN && n_chains * h->ctas_per_chain <= sms;
     CK(cudaDeviceSynchronize());
     CK(cudaGetLastError());
     *out = h;
@@ -1576,7 +1584,7 @@ static int launch_prog(dqmc_handle* h, int mat_id, const PropProg& prog, int rig
         return DQMC_OK;
     }
     PropProg none; none.n = 0;
-    if (!right && !h->fft_L && launch_prop_small(h->d_chains, h->nch, h->maxN, h->max_nb, mat_id, prog, none, h->st)) return DQMC_OK;
+    if (!right && !h->fft_L && !h->spread && launch_prop_small(h->d_chains, h->nch, h->maxN, h->max_nb, mat_id, prog, none, h->st)) return DQMC_OK;
     // dense kinetic steps are GEMMs of their own; the element-wise ops between
     // them run as one propagation kernel per stretch
     PropProg seg; seg.n = 0;
@@ -1595,7 +1603,7 @@ static int launch_prog(dqmc_handle* h, int mat_id, const PropProg& prog, int rig
 
 // G <- L G R: the two passes of a wrap, in one launch where that applies
 static void launch_wrap(dqmc_handle* h, const PropProg& pl, const PropProg& pr) {
-    if (!h->fft_L && launch_prop_small(h->d_chains, h->nch, h->maxN, h->max_nb, 0 /*G*/, pl, pr, h->st)) {
+    if (!h->fft_L && !(h->spread && pl.n + pr.n > 10) && launch_prop_small(h->d_chains, h->nch, h->maxN, h->max_nb, 0 /*G*/, pl, pr, h->st)) {
         tmark(h, DQMC_PROF_PROP_L);
         return;
     }

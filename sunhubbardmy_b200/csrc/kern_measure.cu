@@ -23,10 +23,12 @@
 
 #define MEAS_NT 256
 // Threads per bin (SPLIT) and so bins per CTA (MEAS_NT / SPLIT): a bin's walk over the
-// cells is a chain of loads from the L2.  Two threads a bin fill the device from about
-// 30 chains on (and four gave nothing at 296); with fewer chains eight keep four times
-// as many SMs busy with walks a quarter as long: 66.6 -> 31.8 us a slice for one chain of
-// 256 sites, 154 -> 96 us for 16 of 400 (eight against two).
+// cells is a chain of loads from the L2, and with few chains eight threads a bin keep four times
+// as many SMs busy with walks a quarter as long.  Two threads and eight, us a slice: one chain of
+// 256 sites 66.6 and 31.7, 16 of 256 73.5 and 52.7, 16 of 400 156 and 95, 16 of honeycomb 6 x 6
+// 31.9 and 29.7.  Eight take more CTAs through the set-up of their tables: with 32 chains of
+// honeycomb 6 x 6 31.0 and 34.8, with 64 36.3 and 43.3, though 32 chains of 256 sites still
+// gain (115 and 77).  Up to 16 chains eight were not slower at any lattice timed.
 #define MEAS_SPLIT_MANY 2
 #define MEAS_SPLIT_FEW 8
 

@@ -539,10 +539,12 @@ __global__ void __launch_bounds__(256) k_prop_small(const ChainDev* __restrict__
 }
 
 // L X R in one launch where the chains are small and the programs hold bond and
-// diagonal operators only; returns 0 without launching otherwise.  A wrap of one
-// 16-site chain takes 14.3 + 13.4 us in two launches of the general passes and 15.1 us here
-// (each launch timed by itself), its B product of ten slices 88 against 70 us; a chain
-// of more than 64 sites would keep one SM busy longer than its columns spread over several.
+// diagonal operators only; returns 0 without launching otherwise.  A wrap takes, here and in
+// two launches of the general passes (each launch timed by itself): 14.7 and 27.6 us for one chain
+// of 16 sites, 20.1 and 38.0 of 36, 25.8 and 31.9 of 8 x 8, 36.4 and 37.4 of cubic 4^3 (six bond
+// families); with 296 chains 17.2 and 34.9, 25.9 and 62.1, 34.7 and 95.2, 55.6 and 125.7.  The
+// line lies at 64 sites, where the cubic lattice gains no more: a longer chain would keep
+// one SM busy for longer than its columns spread over several.
 int launch_prop_small(const ChainDev* chains, int nchains, int maxN, int max_nb, int mat_id, const PropProg& pl, const PropProg& pr,
                       cudaStream_t st) {
     if (maxN > PROP_SMALL_N || pl.n + pr.n == 0) return 0;

@@ -92,3 +92,19 @@ def test_bond_updates_with_rejections(sb, oracle, n):
             assert np.array_equal(g.vconf(c), o.vconf())
             assert d["accepted_v"] == o.diag()["accepted_v"]
             assert np.max(np.abs(g.green(c) - o.green())) < 1e-10
+
+
+@pytest.mark.parametrize("case", ["square64", "honeycomb64", "cubic64", "square36", "honeycomb50", "r_cubic48", "chain62"])
+def test_b_products_of_few_and_many_chains(sb, case):
+    """The start-up's G of one chain comes from B products alone: in one launch or in the
+    general passes, by the number of chains and sites, with the same operations on every
+    element, so G of the same field has the same bits in handles of 1, 2 and 160 chains."""
+    lat = {**PROP, "square36": dict(lattice=1, l1=6, l2=6), "honeycomb50": dict(lattice=2, l1=5, l2=5),
+           "r_cubic48": dict(lattice=5, l1=2, l2=2, l3=2, rtd=0.7), "chain62": dict(lattice=3, l1=62, l2=1)}[case]
+    kw = dict(beta=0.6, dtau=0.1, rhub=3.0, mu=0.2, nflr=2, kinetic=0, update=1, hs=1, nwrap=4, nublock=8, **lat)
+    G = []
+    for n in (1, 2, 160):
+        with sb.Dqmc(sb.DqmcParams.make(**kw), n_chains=n, seeds=[sb.test_seed(c) for c in range(n)]) as g:
+            g.sweep_start()
+            G.append(g.green(0))
+    assert np.array_equal(G[0], G[1]) and np.array_equal(G[0], G[2])
