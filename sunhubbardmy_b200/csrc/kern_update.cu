@@ -453,13 +453,14 @@ __global__ void __launch_bounds__(UPD_NT, 2) k_update_flush(const ChainDev* __re
 // rejected one precedes; every CTA takes the decisions for itself.  The flush is two
 // thirds of the kernel with one CTA per chain: a family of honeycomb 12 x 12 takes
 // 2.39 ms for 16 chains with one CTA each, 1.22 ms on teams.
+template <bool TEAM>
 __global__ void __launch_bounds__(UPD_NT, 2) k_vbond_delay(const ChainDev* __restrict__ chains, int nt, int nf, int visit,
                                                            int dir) {
     extern __shared__ double2 dsm[];                  // flush staging
     __shared__ double2 s_ap[2][64], s_bp[2][64];      // A(P_q, m), B(P_q, m) of the current bond
     __shared__ double2 s_mat[4];
     __shared__ int s_pc[2], s_acc;
-    const Team team = this_team();
+    const Team team = TEAM ? this_team() : Team{0, 1};
     const ChainDev& c = chains[blockIdx.x / team.size];
     const ModelDev& md = *c.md;
     if (!md.lwrapv || !c.vconf) return;
@@ -545,9 +546,9 @@ __global__ void __launch_bounds__(UPD_NT, 2) k_vbond_delay(const ChainDev* __res
         }
         if (k > 0 && (k + 2 > nbv || b == lf - 1)) {
             // the last bond rejected: every CTA has read G(P,P) before one stores to G
-            if (!accepted) team.sync();
+            if (TEAM && !accepted) team.sync();
             flush_addto(G, A, B, N, k, dsm, team.rank, team.size);
-            team.sync();
+            if (TEAM) team.sync();      // one CTA: the next bond's barrier
             k = 0;
         }
     }
@@ -561,7 +562,8 @@ __global__ void __launch_bounds__(UPD_NT, 2) k_vbond_delay(const ChainDev* __res
 }
 
 void setup_update() {
-    for (const void* k : {(const void*)k_update_delay<false>, (const void*)k_update_delay<true>, (const void*)k_vbond_delay}) {
+    for (const void* k : {(const void*)k_update_delay<false>, (const void*)k_update_delay<true>, (const void*)k_vbond_delay<false>,
+                          (const void*)k_vbond_delay<true>}) {
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, TEAM_SMEM_MAX);
         cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     }
@@ -574,7 +576,7 @@ int launch_vbond_delay(const ChainDev* chains, int nchains, int nublock, int tea
                        cudaStream_t st) {
     if ((min(nublock, 64) & ~1) < 2) return 0;
     const size_t smem = UpdGemm::SMEM_ELEMS * sizeof(double2);
-    launch_team(k_vbond_delay, nchains, team, smem, st, chains, nt, nf, visit, dir);
+    launch_team(team > 1 ? k_vbond_delay<true> : k_vbond_delay<false>, nchains, team, smem, st, chains, nt, nf, visit, dir);
     return 1;
 }
 
