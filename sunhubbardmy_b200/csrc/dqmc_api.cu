@@ -5,7 +5,7 @@
 // The sweep follows the reference's control flow exactly
 // (src/dqmc_ft_core/dqmc_ft_sweep_b0.f90, dqmc_ft_sweep_0b.f90,
 // dqmc_ft_sweep_start_0b.f90); every chain of a handle is advanced by the same
-// kernel launches (one CTA, or a few, per chain), and a full sweep is captured
+// kernel launches (one CTA per chain, or several), and a full sweep is captured
 // once into a CUDA graph and replayed.
 #include <algorithm>
 #include <cmath>
@@ -1416,7 +1416,7 @@ extern "C" int dqmc_gpu_create(const dqmc_params* params, int n_params, int n_ch
                 d.URs = (double2*)dalloc(h, Nne * z);
                 d.ULTs = (double2*)dalloc(h, Nne * z);
             }
-            d.pw = (double2*)dalloc(h, ((size_t)5 * 32 * ne + 2 * 32 * 32) * z);
+            d.pw = (double2*)dalloc(h, (size_t)3 * 32 * ne * z);
             d.pw_flag = (int*)dalloc(h, 16 * sizeof(int));
             if (!d.UR || !d.ULT || !d.ULRINV || !d.Pst || !d.projR || !d.projLc || !d.logwDV || !d.pw) {
                 dqmc_gpu_destroy(h);

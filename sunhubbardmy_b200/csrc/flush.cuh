@@ -1,14 +1,15 @@
 // The delayed updates' flush, G += A B^T over the first K columns of the
-// N x nb factors A and B, by one CTA on the FP64 tensor pipe (DMMA).
+// N x nb factors A and B, by the CTAs of a chain on the FP64 tensor pipe (DMMA).
 #pragma once
 #include "zgemm.cuh"
 
 typedef GemmBig UpdGemm;
 
 // G += A B^T over the first K columns of the N x nb factors (alpha = beta = 1),
-// the output tiles tile0, tile0 + tstep, ... by this CTA: the accumulators start from the G tile (read
-// while the first A and B stages are in flight) and are stored straight back,
-// so the epilogue needs no shared-memory pass and no second read of G.
+// the output tiles tile0, tile0 + tstep, ... by this CTA: the accumulators start
+// from the G tile (read while the first A and B stages are in flight) and are
+// stored straight back, so the epilogue needs no shared-memory pass and no second
+// read of G.
 DQ_DEV void flush_addto(double2* G, const double2* A, const double2* B, int N, int K, cplx* smem, int tile0, int tstep) {
     typedef UpdGemm Cfg;
     constexpr int BM = Cfg::BM, BN = Cfg::BN, BK = Cfg::BK, FM = Cfg::FM, FN = Cfg::FN;

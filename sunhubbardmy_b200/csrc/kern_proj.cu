@@ -1,5 +1,6 @@
 // Projective (ground-state) DQMC: updates, stabilisation and Green's function
-// of the projector path, one CTA per walker for the sequential parts.
+// of the projector path: one CTA per walker for the update's walk, a team of CTAs
+// (team.cuh) for the QR factorisations.
 //
 // State per walker: UR = B(tau,0) P (N x ne), UL = P^H B(beta,tau) (ne x N,
 // stored transposed as ULT = UL^T, N x ne), ULRINV = (UL UR)^-1 (ne x ne) and
@@ -203,7 +204,7 @@ __global__ void k_tall_copy(const ChainDev* __restrict__ chains, int dst_id, int
 //                UR(A,:) *= 1 + Delta
 //   k_pwin_flush (several CTAs per walker)  ULRINV -= Ut Vt
 // so the window GEMMs use all SMs while the sequential part runs one CTA per
-// walker.  Scratch per walker in pw: Rg (nr x ne), Fg, Gg (nr x nr), Ut, Vt.
+// walker.  Scratch per walker in pw: Rg, Ut and Vt (32 x ne each); F and Gamma stay in shared memory.
 // ---------------------------------------------------------------------------
 struct PUpdSmem {
     double2 F[PW_MAXR * PW_LD];     // F(x, y) of the window at x + y * PW_LD (window-start values)
@@ -240,12 +241,10 @@ DQ_DEV bool pwin(const ChainDev& c, int nf, int w, PWin& p) {
     return true;
 }
 
-DQ_DEV void pw_ptrs(const ChainDev& c, int R, double2*& Rg, double2*& Fg, double2*& Gg, double2*& Ut, double2*& Vt) {
+DQ_DEV void pw_ptrs(const ChainDev& c, int R, double2*& Rg, double2*& Ut, double2*& Vt) {
     const int ne = c.md->ne;
     Rg = c.pw;
-    Fg = Rg + (size_t)R * ne;
-    Gg = Fg + (size_t)R * R;
-    Ut = Gg + (size_t)R * R;
+    Ut = Rg + (size_t)R * ne;
     Vt = Ut + (size_t)ne * R;
 }
 
@@ -256,8 +255,8 @@ __global__ void __launch_bounds__(256) k_pwin_rg(const ChainDev* __restrict__ ch
     PWin p;
     if (!pwin(c, nf, w, p)) return;
     const int N = c.N, ne = c.md->ne;
-    double2 *Rg, *Fg, *Gg, *Ut, *Vt;
-    pw_ptrs(c, p.R, Rg, Fg, Gg, Ut, Vt);
+    double2 *Rg, *Ut, *Vt;
+    pw_ptrs(c, p.R, Rg, Ut, Vt);
     ZGemmArgs ga;   // Rg
     ga.M = p.nr; ga.N = ne; ga.K = ne; ga.alpha = cmk(1, 0); ga.beta = cmk(0, 0);
     ga.A = p.rows ? c.UR : c.UR + p.u0; ga.lda = N; ga.opA = OP_N; ga.arow = p.rows;
@@ -283,8 +282,8 @@ __global__ void __launch_bounds__(256) k_pwin_flush(const ChainDev* __restrict__
     if (!pwin(c, nf, w, p)) return;
     if (c.pw_flag[0] == 0) return;
     const int ne = c.md->ne;
-    double2 *Rg, *Fg, *Gg, *Ut, *Vt;
-    pw_ptrs(c, p.R, Rg, Fg, Gg, Ut, Vt);
+    double2 *Rg, *Ut, *Vt;
+    pw_ptrs(c, p.R, Rg, Ut, Vt);
     ZGemmArgs g;
     g.M = ne; g.N = ne; g.K = p.nr; g.alpha = cmk(-1, 0); g.beta = cmk(1, 0);
     g.A = Ut; g.lda = ne; g.opA = OP_N; g.B = Vt; g.ldb = p.nr; g.opB = OP_N; g.C = c.ULRINV; g.ldc = ne;
@@ -464,8 +463,8 @@ __global__ void __launch_bounds__(256) k_pwin_seq(const ChainDev* __restrict__ c
     }
     const uint32_t* rnd = c.rnd + rnd_off;
     int32_t* cf = bond ? c.vconf + ((size_t)(nt - 1) * md.nn_nf + (nf - 1)) * N : c.conf + (size_t)(nt - 1) * N;
-    double2 *Rg, *Fg, *Gg, *Ut, *Vt;
-    pw_ptrs(c, p.R, Rg, Fg, Gg, Ut, Vt);
+    double2 *Rg, *Ut, *Vt;
+    pw_ptrs(c, p.R, Rg, Ut, Vt);
     for (int x = tid; x < nr; x += nth) S->rows[x] = p.rows ? p.rows[x] : u0 + x;
     __syncthreads();
     {   // F = Rg UL(:,rows) = Rg ULT(rows,:)^T: warp w the columns 16 (w & 1).. and every fourth k step

@@ -1,4 +1,5 @@
-// UDV stabilisation and the equal-time Green's function, one CTA per chain.
+// UDV stabilisation and the equal-time Green's function, a team of CTAs (team.cuh) per
+// chain: up to 16 for a few chains, one for many.
 //
 // Reference: src/dqmc_ft_core/dqmc_ft_stablize_0b_qr.f90 / _b0_qr.f90 (1-61),
 // green_equaltime.f90 (1-107), green_equaltimebb.f90 (1-84), set_phase.f90,
@@ -724,7 +725,7 @@ void launch_dyn_err(const ChainDev* chains, int nchains, cudaStream_t st) {
 
 void launch_zgemm_test(const ChainDev* chains, int nchains, int m, int n, int k, int opa, int opb,
                        int a_id, int b_id, int c_id, double beta_re, cudaStream_t st) {
-    dim3 grid(1, nchains);   // one CTA per chain, as in the stabilisation kernels
+    dim3 grid(1, nchains);   // one CTA per chain
     k_zgemm_test<<<grid, 256, GemmBig::SMEM_ELEMS * sizeof(double2), st>>>(chains, m, n, k, opa, opb, a_id, b_id, c_id, beta_re);
 }
 

@@ -1,4 +1,5 @@
-// Local Hubbard-Stratonovich updates of one time slice, one CTA per chain.
+// Local Hubbard-Stratonovich updates of one time slice, a team of CTAs (team.cuh) per
+// chain, or one CTA where chains are many or small.
 //
 // Reference: src/dqmc_config_u/dqmc_update_delay.f90:1-137 (delayed update),
 // dqmc_update.f90 (fast update) and dqmc_update_submatrix.f90 (submatrix
@@ -437,7 +438,7 @@ __global__ void __launch_bounds__(UPD_NT, 2) k_update_flush(const ChainDev* __re
 }
 
 // The t-V bond field's updates of one family nf at slice nt, delayed
-// (src/dqmc_config_v/dqmc_update_delay.f90:30-112): one CTA per chain, the
+// (src/dqmc_config_v/dqmc_update_delay.f90:30-112): a team of CTAs per chain, the
 // bonds in nnlf_list order.  The accepted rank-2 changes are carried as
 // columns of (A, B), G' = G + A B^T: bond b's 2 x 2 block of G' is
 // G(P,P) + A(P,:) B(P,:)^T (warp 0, lanes over the delayed columns), the ratio

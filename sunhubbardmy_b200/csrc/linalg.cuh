@@ -3,8 +3,9 @@
 // H = I - tau v v^H, v(1) = 1), explicit Q (zungqr), Q^H applied to a matrix,
 // and an upper-triangular solve.  The trailing updates and the triangular
 // solve's off-diagonal blocks run through the DMMA GEMM of zgemm.cuh; the
-// panel factorisation runs in shared memory.  One CTA of 256 threads owns
-// one chain's matrices (leading dimension N, N <= 512).
+// panel factorisation runs in shared memory.  A team of CTAs (team.cuh; one CTA
+// where chains are many) of 256 threads each owns one chain's matrices (leading
+// dimension N, N <= 512).
 #pragma once
 #include "zgemm.cuh"
 #include "team.cuh"

@@ -223,7 +223,6 @@ __device__ void zgemm_cta(const ZGemmArgs& g, int tile0, int tstep, cplx* smem) 
 
 // Default tile configurations (256 threads).
 typedef ZGemmCfg<64, 64, 16, 2, 4> GemmBig;     // square-ish products
-typedef ZGemmCfg<32, 64, 16, 2, 4> GemmMid;     // panels with M <= 32
 typedef ZGemmCfg<16, 128, 16, 1, 8> GemmWide;   // M = 16 rows (reflector blocks)
 typedef ZGemmCfg<16, 64, 16, 1, 8> Gemm16x64;   // M = 16 rows, up to 64 columns
 // narrow column chunks and single tiles of a matrix that a team of CTAs shares
@@ -265,9 +264,4 @@ DQ_DEV void zgemm_tile(const ZGemmArgs& g, int cls, int t, cplx* smem) {
     case ZT_32x32: zgemm_cta<Gemm32x32>(g, t, big, smem); break;
     default: zgemm_cta<GemmBig>(g, t, big, smem); break;
     }
-}
-// every tile, by the whole CTA, in the best-fitting shape
-DQ_DEV void zgemm_fit(const ZGemmArgs& g, cplx* smem) {
-    const int cls = zt_pick(g.M, g.N), nt = zt_tiles(cls, g.M, g.N);
-    for (int t = 0; t < nt; ++t) zgemm_tile(g, cls, t, smem);
 }
