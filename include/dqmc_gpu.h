@@ -20,7 +20,11 @@
  *    thread.  The caller owns every host buffer; the library owns all device
  *    state.
  *  - A handle holds n_chains independent Markov chains (the reference's MPI
- *    ranks) that are advanced together, one CTA per chain.
+ *    ranks) that are advanced together, by a cluster of up to 16 CTAs per chain where
+ *    chains are few and by one CTA per chain where they are many.  What the other
+ *    chains are does not touch a chain, but how many there are sets the order of some
+ *    sums: the same chain in handles of other sizes agrees to rounding, and may
+ *    part at an accept decision that is tied to rounding (near_ties of dqmc_diag).
  */
 #ifndef DQMC_GPU_H
 #define DQMC_GPU_H

@@ -1,9 +1,9 @@
 """Batched chains of uneven sizes and the delay-depth autotuner.
 
-A handle advances many independent chains in one launch per kernel (one CTA
-per chain), the GPU form of the reference's one-chain-per-MPI-rank runs
-(src/dqmc_main.f90).  Chains may have different lattice sizes as long as they
-share ltrot, nwrap, the lattice kind and the kinetic propagator.
+A handle advances many independent chains in one launch per kernel (a cluster of
+CTAs per chain, or one CTA where chains are many), the GPU form of the reference's
+one-chain-per-MPI-rank runs (src/dqmc_main.f90).  Chains may have different
+lattice sizes as long as they share ltrot, nwrap, the lattice kind and the kinetic propagator.
 
 The flush depth (nublock: accepted flips folded into G by one tensor-core
 GEMM) trades GEMM efficiency against the cost of building longer delayed
@@ -16,8 +16,8 @@ SMs of the small chains idle while the N = 288 CTAs finish.  `ChainGroup`
 instead gives each size class (split into a few handles) its own stream
 (dqmc_gpu_sweeps_multi): the small classes' kernels fill the SMs that the
 large class's long kernels leave free.  Chains are independent and each
-keeps its seed, so a group gives the same fields, Green's functions and bins
-as one handle of all its chains.
+keeps its seed, so a group gives the same fields, and to rounding the same Green's
+functions and bins, as one handle of all its chains.
 """
 from __future__ import annotations
 
