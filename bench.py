@@ -519,7 +519,7 @@ def gpu_arm(args, rank: int, world: int, local_rank: int) -> None:
         trf = os.path.join(ROOT, "profiles", "traffic.json")
         if os.path.exists(trf):
             tr = json.load(open(trf)).get(roof["kernel"])
-            if tr:
+            if tr and tr["workload"] == args.workload and tr["chains"] == C:
                 roof["traffic"] = tr["bytes_per_chain"] * C
                 roof["traffic_note"] = tr.get("note", "")
         result = {
@@ -622,12 +622,6 @@ def proj_roofline_and_line(args, g, p, Ns, ms, value, per_step, world, workload,
     from sunhubbardmy_b200.autotune import ChainGroup
     if isinstance(g, ChainGroup):
         roof["timing"] += f" (one handle of all {len(Ns)} walkers, after one warm-up sweep)"
-    trf = os.path.join(ROOT, "profiles", "traffic.json")
-    if os.path.exists(trf):
-        tr = json.load(open(trf)).get(roof["kernel"])
-        if tr:
-            roof["traffic"] = tr["bytes_per_chain"] * C
-            roof["traffic_note"] = tr.get("note", "")
     result = {
         "metric": METRIC, "value": value, "unit": "updates/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True, "scaling": "weak",
