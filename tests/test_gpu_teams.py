@@ -89,7 +89,7 @@ def test_forced_flips(sb, l, n):
 
 
 # sites of a chain and chains of each handle
-GROUPS = {"16x4": [(100, 4)] * 16, "4x20": [(130, 20)] * 4, "2x74": [(98, 74)] * 2, "sizes": [(72, 12), (162, 8), (36, 12)],
+GROUPS = {"16x4": [(100, 4)] * 16, "4x20": [(130, 20)] * 4, "2x74": [(98, 74)] * 2, "3x74": [(98, 74)] * 3, "sizes": [(72, 12), (162, 8), (36, 12)],
           "2x1": [(130, 1)] * 2}
 
 
